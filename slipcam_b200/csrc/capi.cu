@@ -24,8 +24,6 @@
 #include <emmintrin.h>
 #endif
 
-#include <cudaTypedefs.h>
-
 #include "../../include/slipcam_b200.h"
 #include "corr_fft.cuh"
 #include "corr_big.cuh"
@@ -336,38 +334,8 @@ void launch_corr_big(const CorrArgs &a, float2 *, cudaStream_t s)
     corr_big_cluster_kernel<kBigN, kThreads><<<unsigned(2 * clusters), kThreads, BigClusterGeo<kBigN>::smem_bytes, s>>>(a);
 }
 
-// cuTensorMapEncodeTiled, from the driver through the runtime (no link against libcuda)
-PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
-{
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    if (!fn) {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q{};
-        CK(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q));
-        if (q != cudaDriverEntryPointSuccess || !p) fail(B200_ERUNTIME, "cuTensorMapEncodeTiled is not available");
-        fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    }
-    return fn;
-}
-
-// the variance denominators of a group (nf frames of h x w floats) as a 3-D TMA tensor, box
-// tc_box_width(M) x M x 1
-CUtensorMap dinv_map(const float *dinv, int h, int w, int dpitch, int nf, int M)
-{
-    CUtensorMap m{};
-    const cuuint64_t dims[3] = {cuuint64_t(w), cuuint64_t(h), cuuint64_t(nf)};
-    const cuuint64_t strides[2] = {cuuint64_t(dpitch) * 4, cuuint64_t(dpitch) * h * 4};
-    const cuuint32_t box[3] = {cuuint32_t(tc_box_width(M)), cuuint32_t(M), 1};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    const CUresult r = tensor_map_encoder()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float *>(dinv), dims, strides,
-                                            box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) fail(B200_ERUNTIME, "cuTensorMapEncodeTiled failed (" + std::to_string(int(r)) + ")");
-    return m;
-}
-
 template <int N>
-void launch_corr_tc(const CorrArgs &a, const uint4 *dtab, int *status, const CUtensorMap *dmap, cudaStream_t s)
+void launch_corr_tc(const CorrArgs &a, const uint4 *dtab, int *status, cudaStream_t s)
 {
     static bool done[64] = {};
     int dev = 0;
@@ -378,7 +346,7 @@ void launch_corr_tc(const CorrArgs &a, const uint4 *dtab, int *status, const CUt
     }
     const int pairs = a.nwin * a.nf;
     const int grid = std::min(pairs, num_sms());
-    corr_tc_kernel<N><<<unsigned(grid), kTcThreads, TcGeo<N>::smem_bytes, s>>>(a, dtab, status, dmap);
+    corr_tc_kernel<N><<<unsigned(grid), kTcThreads, TcGeo<N>::smem_bytes, s>>>(a, dtab, status);
 }
 
 // the exact tensor-core form: one persistent CTA per SM over the groups of F frames of a window
@@ -402,15 +370,18 @@ void launch_corr_i8(const CorrArgs &a, const uint8_t *refwin, const int *sref, i
         corr_i8_kernel<false><<<unsigned(grid), kI8Threads, g.smem, s>>>(x);
 }
 
+// The geometries the tensor-core form takes, by FFT size and surface side: those whose box of variance
+// denominators (rows of M + 3 floats rounded up to 4) fits the larger of its chip and S5 operands, with
+// NO columns of correlation beside 512 - NO of other accumulators. The kernel itself holds every M up to
+// 128; the others stay on the FP32 form, whose accuracy their callers have.
 template <int N>
 bool tc_fits_n(int M)
 {
-    // the box of variance denominators (X region), and the S5 result in the top NO TMEM columns
-    // clear of every other stage's accumulators
-    using G = TcGeo<N>;
+    constexpr int KP = TcGeo<N>::KP, T1 = (N + 127) / 128;
+    constexpr size_t room = std::max<size_t>(size_t(N) * N * 2, size_t(16) * (2 * KP) * 16);
     const int NO = (M + 15) / 16 * 16;
-    const int used = std::max({2 * G::KP * G::T1, 2 * N, 2 * NO});
-    return size_t(tc_box_width(M)) * M * 4 <= G::X_BYTES && used + NO <= int(G::TMEM_COLS);
+    const int used = std::max({2 * KP * T1, 2 * N, 2 * NO});
+    return size_t((M + 3 + 3) / 4 * 4) * M * 4 <= room && used + NO <= 512;
 }
 
 // whether the tensor-core kernel holds this geometry: FFT size up to 160, up to 128 shifts per axis
@@ -510,7 +481,6 @@ struct b200_handle {
     DevBuf<float> d_cdinv;
     DevBuf<uint16_t> d_dtab;     // the FP16 DFT matrices of the tensor-core form
     DevBuf<int> d_status;        // device status word (3: a tensor-core wait gave up)
-    DevBuf<CUtensorMap> d_tmaps; // TMA maps of the three denominator tables: slot 0, slot 1, device path
     DevBuf<float> d_coarse;      // coarse tracking: one frame's surfaces and four outputs
     DevBuf<double> d_cpeaks;     // coarse tracking: one frame's peaks
     cudaEvent_t coarse_ev[6] = {};  // coarse tracking: tables ready (2), tables consumed (2), call start, end
@@ -549,10 +519,11 @@ struct b200_handle {
     int64_t sat_size() const { return int64_t(height + 1) * (width + 1); }
     int64_t pixels() const { return int64_t(height) * width; }
     int dpitch() const { return (width + 3) & ~3; }                  // rows of 16-byte multiples
+    // rows that the tensor-core kernel may read (and ignore) past a surface's last
+    int64_t dinv_pad() const { return 8 * int64_t(dpitch()); }
     int64_t dinv_size() const { return int64_t(height) * dpitch(); }
 
-    // the host path's two slots (device and page-locked host buffers, events, the TMA maps of their
-    // tables), allocated by the first host-path call: device-path callers never pay for them
+    // the host path's two slots (device and page-locked host buffers, events), allocated by the first host-path call: device-path callers never pay for them
     void ensure_slots()
     {
         if (slots_ready) return;
@@ -561,7 +532,7 @@ struct b200_handle {
             s.frames.alloc(G * height * fpitch);
             s.sat.alloc(G * sat_size());
             s.sat2.alloc(G * sat_size());
-            s.dinv.alloc(G * dinv_size());
+            s.dinv.alloc(G * dinv_size() + dinv_pad());
             s.gross.alloc(2 * P);
             s.out.alloc(7 * P);
             s.hframes.alloc(G * height * fpitch);
@@ -570,27 +541,17 @@ struct b200_handle {
             if (!s.in) CK(cudaEventCreateWithFlags(&s.in, cudaEventDisableTiming));
             if (!s.done) CK(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming));
         }
-        if (tc_ok) {
-            const CUtensorMap maps[2] = {dinv_map(slot[0].dinv.p, height, width, dpitch(), int(G), M),
-                                         dinv_map(slot[1].dinv.p, height, width, dpitch(), int(G), M)};
-            CK(cudaMemcpy(d_tmaps.p, maps, sizeof(maps), cudaMemcpyHostToDevice));
-        }
         slots_ready = true;
     }
 
-    // the device path's tables for `group` frames (and the TMA map of its denominators), allocated
-    // by the first device-path call: coarse tracking and the host path never pay for them
+    // the device path's tables for `group` frames, allocated by the first device-path call: coarse tracking and the host path never pay for them
     void ensure_tables()
     {
         if (!d_sat.p) {
             const size_t G = size_t(group);
             d_sat.alloc(G * sat_size());
             d_sat2.alloc(G * sat_size());
-            d_dinv.alloc(G * dinv_size());
-            if (tc_ok) {
-                const CUtensorMap m = dinv_map(d_dinv.p, height, width, dpitch(), int(G), M);
-                CK(cudaMemcpy(d_tmaps.p + 2, &m, sizeof(m), cudaMemcpyHostToDevice));
-            }
+            d_dinv.alloc(G * dinv_size() + dinv_pad());
         }
         ensure_exact(d_bstat, d_peaks, d_queue);
     }
@@ -734,10 +695,7 @@ struct b200_handle {
             launch_corr_i8(a, d_refwin.p, d_sref.p, d_status.p, i8g, s);
         } else if (arith == B200_FORM_TC) {
             const uint4 *dt = reinterpret_cast<const uint4 *>(d_dtab.p);
-            const int mi = dinv == slot[0].dinv.p ? 0 : dinv == slot[1].dinv.p ? 1 : 2;
-            if (mi == 2 && dinv != d_dinv.p) fail(B200_EINVAL, "no TMA map for this denominator table");
-            const CUtensorMap *dm = d_tmaps.p + mi;
-            B200_DISPATCH_TC(N, launch_corr_tc, a, dt, d_status.p, dm, s);
+            B200_DISPATCH_TC(N, launch_corr_tc, a, dt, d_status.p, s);
         } else if (N == kBigN) {
             launch_corr_big(a, d_big.p, s);
         } else if (N == 192) {
@@ -838,7 +796,7 @@ void upload_reference(b200_handle *h, const uint8_t *dframe, int pitch, cudaStre
     CK(cudaGetLastError());
     h->launches += 1;
     if (h->tc_ok) {
-        spec_tc_kernel<<<unsigned(4 * num_sms()), 256, 0, s>>>(h->d_spec.p, h->d_spec_tc.p, h->N, h->nwin);
+        spec_tc_kernel<<<unsigned(4 * num_sms()), 256, 0, s>>>(h->d_spec.p, h->d_norm.p, h->W, h->d_spec_tc.p, h->N, h->nwin);
         CK(cudaGetLastError());
         h->launches += 1;
     }
@@ -889,16 +847,14 @@ DiffArgs diff_args(b200_handle *h, const float *frames, int n, int pitch, const 
 
 void b200::tc_dft_table(int N, uint16_t *out)
 {
-    const uint32_t sbo = uint32_t(N / 8) * 128u, bytes = uint32_t(N / 8) * sbo;
-    for (int part = 0; part < 2; ++part)
-        for (int r = 0; r < N; ++r)
-            for (int c = 0; c < N; ++c) {
-                double cc = 0.0, sn = 0.0;
-                cs2pi(long(r) * c, N, cc, sn);
-                const __half hv = __float2half_rn(float(part == 0 ? cc : -sn));
-                const uint32_t off = part * bytes + tc::k_major_offset(r, c, sbo, 128);
-                out[off / 2] = __half_as_ushort(hv);
-            }
+    for (int r = 0; r < tc_rt(N); ++r)
+        for (int c = 0; c < N; ++c) {
+            double cc = 0.0, sn = 0.0;
+            cs2pi(long(r < N / 2 ? r : r - N / 2) * c, N, cc, sn);
+            double v = r < N / 2 ? cc : r <= N ? -sn : 0.0;
+            if (r == N / 2) v = c % 2 ? -1.0 : 1.0;   // the Nyquist row, where S's row 0 would be
+            out[tc_table_offset(N, r, c) / 2] = __half_as_ushort(__float2half_rn(float(v)));
+        }
 }
 
 extern "C" {
@@ -964,7 +920,7 @@ int b200_create(const b200_params *p, int device, b200_handle **out)
         CK(cudaMemset(h->d_status.p, 0, sizeof(int)));
         h->tc_ok = tc_fits(N, h->M);
         if (h->tc_ok) {
-            std::vector<uint16_t> dt(2 * size_t(N) * N);
+            std::vector<uint16_t> dt(size_t(tc_rt(N)) * N);
             tc_dft_table(N, dt.data());
             h->d_dtab.alloc(dt.size());
             h->d_spec_tc.alloc(size_t(h->nwin) * (N / 2) * tc_kp(N));
@@ -976,8 +932,6 @@ int b200_create(const b200_params *p, int device, b200_handle **out)
             h->d_refwin.alloc(size_t(h->nwin) * h->W * h->W);
             h->d_sref.alloc(h->nwin);
         }
-        // the maps of the two slots and of the device path's table are written when those are allocated
-        if (h->tc_ok) h->d_tmaps.alloc(3);
         h->form = auto_form(h);
         *out = h;
         g_create_error.clear();

@@ -1,21 +1,55 @@
 // corr_tc.cuh -- the tensor-core form: the 2-D DFTs of the correlation as dense DFT-matrix GEMMs
-// on tcgen05 (FP16 operands, FP32 accumulation in TMEM), one (window, frame) pair at a time per
-// persistent CTA. With D = [w_N^{rc}] (Dr = cos, Di = -sin, N x N, resident in shared memory as
-// FP16) every stage is a GEMM whose fixed operand is a block of Dr or Di:
+// on tcgen05 (FP16 operands, FP32 accumulation in TMEM), (window, frame) pairs streaming through a
+// persistent CTA per SM. With C = [cos(2 pi r c / N)] and S = [-sin(2 pi r c / N)], FP16, resident in
+// shared memory, a pair is
 //
-//   S1  Y  = X Dr|Di          rows i (chip rows), K = j, N = kappa (Re | Im)     X = chip - round(mean)
-//   S2  Z^T = Y^T D            rows kappa, K = (Re|Im, i), N = (Re|Im, ky)        A2 MN-major from S1's rows
-//   S3  P = Z conj(R) 2^-s     per thread (one kappa row), R the resident reference spectrum
-//   S4  Q^T = P^T conj(D)      rows kappa, K = (Re|Im, ky), N = (Re|Im, u < M)    A4 K-major from S3's rows
-//   S5  c^T = [Dr|Di] (w Q)    rows v, K = (Re|Im, kappa), N = u                  B5 MN-major from S4's rows
+//   S1  Yr^T = C X^T, Yi^T = S X^T       rows kappa (frequency across), columns i   X = chip - round(mean)
+//   S2  [P1|P3] = Yr [C|S]^T,            rows kappa, columns r = 0 .. N/2 - 1 (frequency down) of each:
+//       [P4|P2] = Yi [C|S]^T             the spectrum at ky = r is (P1 - P2, P3 + P4), at N - r (P1 + P2, P4 - P3)
+//   S3  P = Z conj(R) 2^-s               per thread (one kappa row), R the resident reference spectrum
+//   S4  [Pr C|Pr S], [Pi C|Pi S]         rows kappa, columns u = 0 .. N/2 - 1, as S2: Q at u and at N - u
+//   S5  c^T = [C|S] (w Q)                rows v, columns u < M, w the Hermitian weights
 //
-// then the normalization by the variance denominators, the argmax and the FP64 peak epilogue of
-// the FP32 form. Each stage writes the next stage's operand straight from its TMEM rows: a thread
-// owns one accumulator row and stores it as 16-byte chunks, in the major order the next GEMM reads.
+// then the normalization by the variance denominators, the argmax and the peak's values. C at N - r is
+// C at r and S changes sign, so columns r < N/2 give the whole of S2's and S4's results in half the
+// products, and one table serves every stage: its rows are C 0 .. N/2 - 1, then the Nyquist row (-1)^c,
+// then S 1 .. N/2. The Nyquist row is C's row N/2 and stands where S's row 0 (zero) would: S1 and S5 zero
+// what it touches as S's, and as a column of P2 and P3 it is the spectrum at ky = N/2 that r < N/2 lacks
+// (the same for u = N/2). As A the table is read K-major in S1 and MN-major in S5, as B (its first N rows,
+// C and S at once, so that an MMA is N columns wide and the tensor core, not the operands' 128 bytes of
+// shared memory a cycle, bounds it: 80 cycles at N = 160) K-major in S2 and S4.
+//
+// Seven roles, linked by mbarriers (one completion per pair and barrier):
+//   control   issues every MMA; the order S4(p), S1(p + 1) Yr, S5(p), S1(p + 1) Yi, S2(p + 1) keeps the
+//             tensor core busy while the drains run
+//   drain     12 warps, four per TMEM quadrant 0-2 (kappa < 96): Y to the FP16 operand of S2, S3, Q to
+//             the FP16 operand of S5
+//   epilogue  8 warps: c of the last pair from TMEM, normalized, its argmax and patch sums
+//   gather    8 warps: the next chip
+//   setup     works out the pairs ahead, 32 at a time, one per lane
+//   relay     waits for the MMAs of each stage and wakes the warps that go on with them at a hardware
+//             barrier (28 warps polling mbarriers took most of the load-store unit's cycles)
+//   spectrum  brings R in by bulk copies, a ring of 5 x 8 frequencies, four of them in S5's operand's
+//             bytes, which are free from S5(p) to S4(p + 1): loads to registers would pass through the
+//             few KB of L1 that this much shared memory leaves
+// An MMA here takes nine tenths of the SM's shared-memory bandwidth, so whatever else goes through it
+// (stores of operands, copies, loads through L1) all but waits while MMAs run: S2 starts when both halves
+// of its operand are in.
+//
+// Measured at 720p, window 64, search 48 (N = 160, 39,200 pairs a launch): 2.16 ms, 15,500 cycles a pair
+// and SM, where one role after the other in the same 12 warps took 3.96 ms; N = 96 (window 48, search 24)
+// 10,600 cycles. The MMAs are 5,500 of them. What bounds a pair is the instruction cache: the roles' code,
+// each executed once a pair, comes at 10 to 16 cycles an instruction (more warps on the same code helped,
+// unrolled copies of it hurt: 179 KB of code took 2.39 ms, rolled into 68 KB the same design 2.16 ms),
+// and the chain S4, Q's drain, S5, Yi, its drain, S2, S3 with the epilogue's hold on c beside it.
+//
+// TMEM columns: Q [0, 2N), then c [0, NO) and Yi [NO, NO + N) once it is drained; Yr [2N, 3N); S2's
+// products replace Y where it was.
+//
 // Power-of-two scales keep every FP16 operand in range: |X| <= 255, |Y| <= 255 N, the reference
 // spectrum is scaled by 2^-e with 2^e > W * norm >= max |R|, P by 2^-8 (|P| <= N^2 255 2^-8 < 2^15
-// for N <= 160) and w Q by 2^-9. Fixed-size tensor-core tiles: rows beyond the data (chip rows >= N, kappa rows
-// >= KP, output rows >= M) read whatever follows in shared memory and their results are ignored.
+// for N <= 160) and w Q by 2^-9. Fixed-size tensor-core tiles: rows beyond the data (kappa rows >= KP,
+// output rows >= M) read whatever follows in shared memory and their results are ignored.
 #pragma once
 
 #include <cuda.h>
@@ -30,42 +64,41 @@ constexpr uint32_t cmax(uint32_t a, uint32_t b) { return a > b ? a : b; }
 
 // the frequency rows kappa of a real N-point row transform (N / 2 + 1), padded to 16
 __host__ __device__ constexpr int tc_kp(int N) { return (N / 2 + 1 + 15) / 16 * 16; }
+// the rows of the table: C 0 .. N/2 - 1, the Nyquist row, S 1 .. N/2, zeros up to S's row KP - 1
+__host__ __device__ constexpr int tc_rt(int N) { return N / 2 + tc_kp(N); }
+// element (r, c) of the table, bytes: column groups of 8, rows of 16 bytes
+B200_HD uint32_t tc_table_offset(int N, int r, int c)
+{
+    return uint32_t(c / 8) * uint32_t(tc_rt(N)) * 16u + uint32_t(r) * 16u + uint32_t(c % 8) * 2u;
+}
 
 template <int N>
 struct TcGeo {
     static constexpr int NH = N / 2 + 1;                            // frequencies of a real row
     static constexpr int KP = tc_kp(N);                             // kappa rows, padded
-    static constexpr int T1 = (N + 127) / 128;                      // row tiles of S1
-    static constexpr uint32_t SBO_D = uint32_t(N / 8) * 128u;       // Dr, Di, X: K-major rows of N
-    static constexpr uint32_t SBO_A = uint32_t(2 * N / 8) * 128u;   // A2 (MN-major), A4 (K-major): K = 2N
-    static constexpr uint32_t SBO_B5 = uint32_t(2 * KP / 8) * 128u; // B5 (MN-major): K = 2 KP
+    static constexpr int RT = tc_rt(N);
+    static constexpr uint32_t SBO_T = uint32_t(RT) * 16u;           // the table's column groups
+    static constexpr uint32_t T_BYTES = uint32_t(N / 8) * SBO_T;
+    static constexpr uint32_t SBO_X = uint32_t(N / 8) * 128u;       // X: K-major rows of N
+    static constexpr uint32_t SBO_A = uint32_t(2 * N / 8) * 128u;   // Y, P: K-major rows (Re | Im, i or ky)
+    static constexpr uint32_t SBO_B5 = uint32_t(2 * KP / 8) * 128u; // w Q (MN-major): K = 2 KP
     static constexpr uint32_t A_BYTES = uint32_t(KP / 8) * SBO_A;
-    static constexpr uint32_t X_BYTES = cmax(uint32_t(N / 8) * SBO_D, 16u * SBO_B5);
-    static constexpr uint32_t D_BYTES = uint32_t(N / 8) * SBO_D;
-    static constexpr uint32_t OFF_X = A_BYTES, OFF_DR = OFF_X + X_BYTES, OFF_DI = OFF_DR + D_BYTES;
-    static constexpr uint32_t END = OFF_DI + D_BYTES;
-    // the furthest byte a full 128-row tile reads
-    static constexpr uint32_t READ_END = cmax(cmax(16u * SBO_A, OFF_X + uint32_t(T1) * 16u * SBO_D),
-                                              cmax(OFF_DI + 16u * SBO_D, END));
+    static constexpr uint32_t X_BYTES = uint32_t(N / 8) * SBO_X;
+    static constexpr uint32_t B5_BYTES = 16u * SBO_B5;              // = 4 slots of R_BYTES
+    static constexpr uint32_t R_BYTES = 8u * uint32_t(KP) * 16u;    // 8 frequencies (and their mirrors) of R
+    static constexpr uint32_t OFF_A = T_BYTES, OFF_X = OFF_A + A_BYTES, OFF_B5 = OFF_X + X_BYTES;
+    static constexpr uint32_t END = OFF_B5 + 5u * R_BYTES;           // the ring: B5 and one slot more
+    // the furthest byte a full 128-row tile reads: rows of A, table rows (S1), table columns (S5)
+    static constexpr uint32_t READ_END =
+        cmax(cmax(END, OFF_A + 16u * SBO_A), cmax(uint32_t(N / 8 - 1) * SBO_T + uint32_t(N / 2 + 128) * 16u, 16u * SBO_T + uint32_t(N / 2) * 16u));
     static constexpr size_t smem_bytes = READ_END;
     static constexpr uint32_t TMEM_COLS = 512;
-    static_assert(KP <= 128 && T1 * 2 * KP <= 512 && 2 * N <= 512, "TMEM or tile bounds");
-    static_assert(READ_END <= 227 * 1024, "shared memory");
+    static constexpr int NR = N / 16;   // chunks of 8 frequencies (S3) or rows u (S5's operand) and their mirrors
+    static_assert(KP <= 96 && 3 * N <= 512, "TMEM or tile bounds");
+    static_assert(READ_END <= 225 * 1024 + 512 && 4 * R_BYTES == B5_BYTES, "shared memory");
 };
 
 #ifdef __CUDACC__
-
-__device__ __forceinline__ uint4 pack8(const float *v, float s)
-{
-    uint4 r;
-    __half2 h0 = __floats2half2_rn(v[0] * s, v[1] * s), h1 = __floats2half2_rn(v[2] * s, v[3] * s);
-    __half2 h2 = __floats2half2_rn(v[4] * s, v[5] * s), h3 = __floats2half2_rn(v[6] * s, v[7] * s);
-    r.x = *reinterpret_cast<uint32_t *>(&h0);
-    r.y = *reinterpret_cast<uint32_t *>(&h1);
-    r.z = *reinterpret_cast<uint32_t *>(&h2);
-    r.w = *reinterpret_cast<uint32_t *>(&h3);
-    return r;
-}
 
 __device__ __forceinline__ uint4 pack8(const float *v)
 {
@@ -79,26 +112,64 @@ __device__ __forceinline__ uint4 pack8(const float *v)
     return r;
 }
 
-// kTcCompute compute warps, kTcParts per TMEM lane quadrant (warps w, w + 4, ... own the same 32
-// accumulator rows and split their columns), and a control warp whose first thread issues the MMAs
-// and the TMA copies, polls their completion and does the per-pair scalar work, so that no compute
-// warp waits behind the tensor core's issue queue
-constexpr int kTcCompute = 12;
-constexpr int kTcParts = kTcCompute / 4;
-constexpr int kTcThreads = 32 * (kTcCompute + 1);
-constexpr int kTcCtrl = 32 * kTcCompute;   // the control thread
-
-// the MMAs of the current phase have completed: the control thread polls the mbarrier, the others
-// wait at the barrier; false (for all threads) if the poll gave up or any thread passes also_failed
-__device__ __forceinline__ bool tc_wait_all(uint64_t *mbar, uint32_t &phase, bool also_failed = false)
+// two floats in one register pair: one instruction works on both, each rounded as the scalar one rounds
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { f32x2 d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) { f32x2 d; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
+__device__ __forceinline__ f32x2 neg2(f32x2 a) { return a ^ 0x8000000080000000ull; }
+__device__ __forceinline__ f32x2 both(float x) { const uint32_t b = __float_as_uint(x); return (f32x2(b) << 32) | b; }
+// the j-th pair of registers read from TMEM
+template <int R>
+__device__ __forceinline__ f32x2 pair2(const uint32_t (&r)[R], int j) { return (f32x2(r[2 * j + 1]) << 32) | r[2 * j]; }
+// the two rounded to FP16, in order and exchanged
+__device__ __forceinline__ uint32_t half2_bits(f32x2 a)
 {
-    bool ok = true;
-    if (threadIdx.x == kTcCtrl) ok = tc::mbar_wait(mbar, phase);
-    phase ^= 1u;
-    const bool failed = __syncthreads_or(!ok || also_failed);
-    tc::fence_after_sync();
-    return !failed;
+    const __half2 h = __floats2half2_rn(__uint_as_float(uint32_t(a)), __uint_as_float(uint32_t(a >> 32)));
+    return *reinterpret_cast<const uint32_t *>(&h);
 }
+__device__ __forceinline__ uint32_t half2_swapped(f32x2 a)
+{
+    const __half2 h = __floats2half2_rn(__uint_as_float(uint32_t(a >> 32)), __uint_as_float(uint32_t(a)));
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+
+// read-only loads that stay where they are written, so that what is fetched ahead of a wait is in
+// flight during it (the compiler moves a plain __ldg down to its first use)
+__device__ __forceinline__ float ldg_here(const float *p)
+{
+    float v;
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+
+__device__ __forceinline__ float4 ldg_here(const float4 *p)
+{
+    float4 v;
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+
+__device__ __forceinline__ uint4 ldg_here(const uint4 *p)
+{
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
+// the warps of each role, 32 in all (eight per SM partition, which is also the TMEM quadrant a warp
+// reads): of 0-15 the first three of each four drain; the others, whose quadrant has nothing to drain,
+// are control (3), the spectrum's copies (7), the pairs' setup (11) and the relay (15); 16-23 epilogue,
+// 24-31 gather
+constexpr int kTcParts = 4;                 // drain warps per quadrant
+constexpr int kTcDrain = 3 * kTcParts;
+constexpr int kTcControl = 3, kTcFetch = 7, kTcSetup = 11, kTcRelay = 15;
+constexpr int kTcEpi = 8, kTcGather = 8;
+constexpr int kTcThreads = 1024;
+constexpr int kTcSlots = 5;                 // of the spectrum's ring: 8 frequencies each
+// the hardware barriers on which the relay wakes the drain warps and (C) the epilogue warps
+constexpr int kTcWake = 2, kTcWakeQ = 2, kTcWakeYr = 3, kTcWakeC = 4, kTcWakeYi = 5, kTcWakeZ = 6;
 
 // 4 pixels (a little-endian word) minus the same offset, as two exact FP16 pairs: a byte b placed
 // under the exponent byte 0x64 reads as the half 1024 + b, and 1024 + b - (1024 + m) is exact
@@ -112,680 +183,875 @@ __device__ __forceinline__ void bytes_to_half(uint32_t word, __half2 off, uint32
     hi = *reinterpret_cast<uint32_t *>(&hb);
 }
 
-// shared-memory operands written by this thread become visible to the tensor core
-__device__ __forceinline__ void tc_publish()
+// one (window, frame) pair of the tensor-core kernel, as the setup warp works it out ahead of time
+struct PairSetup {
+    int64_t q;              // the output index f * nwin + k
+    int k, f, gy, gx;       // window, frame, gross offset
+    int sy, sx, mean;       // the chip's top-left corner and its rounded mean
+    float scale;            // of c: undoes the power-of-two scales, the transform's N^2 and the norm
+    bool end;               // no pair: the roles leave
+    uint32_t seq;           // which pair of the CTA, from 1 (entries are read before a barrier says so)
+};
+
+// the mbarriers of the tensor-core kernel, one completion of each per pair
+struct TcBars {
+    uint64_t xfull, xfree;          // the chip is in X; S1 has read it
+    uint64_t afull;                 // S2's operand is in shared memory
+    uint64_t pfull, b5full;         // S4's, S5's
+    uint64_t cfree;                 // the correlation is read
+    uint64_t stage[5];              // in TMEM: Q (S4), Yr (S1), c (S5), Yi (S1), Z (S2)
+    uint64_t rfull[kTcSlots], rfree[kTcSlots];   // a slot of the reference spectrum's ring, per use of the slot
+};
+
+// wait for the phase `parity` of the mbarrier; false if another role gave up or two seconds went by
+// (the abort flag is then set for the others). The polling is one function for all roles: what they
+// execute has to fit the SM's instruction cache together.
+__device__ __noinline__ bool tc_wait_poll(uint64_t *bar, uint32_t parity, volatile int *abort)
+{
+    uint64_t t0, t1;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+    for (;;) {
+        if (tc::mbar_wait(bar, parity, 16)) return true;
+        if (*abort) return false;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
+        if (t1 - t0 > 2000000000ull) {
+            *abort = 1;
+            return false;
+        }
+    }
+}
+
+__device__ __forceinline__ bool tc_wait(uint64_t *bar, uint32_t parity, volatile int *abort)
+{
+    return tc::mbar_wait(bar, parity, 1) || tc_wait_poll(bar, parity, abort);
+}
+
+// the same for a whole warp, the answer uniform
+__device__ __forceinline__ bool tc_wait_warp(uint64_t *bar, uint32_t parity, volatile int *abort)
+{
+    const bool ok = __all_sync(0xffffffffu, tc_wait(bar, parity, abort));
+    tc::fence_after_sync();
+    return ok;
+}
+
+// The relay's wake-up and its other side: `threads` threads at hardware barrier id, 32 of them the
+// relay's. good holds how many of the barrier's events have come about: the relay counts one before the
+// wake-up or, once a wait gave up, never again, so all who are woken for event n take the same decision
+// (and all leave before they would meet at another barrier).
+__device__ __forceinline__ void wake(int id, int threads, volatile uint32_t *good, uint32_t n, bool ok, int lane)
+{
+    if (ok && lane == 0) *good = n + 1;
+    __syncwarp();
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+template <int ID>
+__device__ __forceinline__ bool woken(int threads, const volatile uint32_t *good, uint32_t n)
+{
+    asm volatile("bar.sync %0, %1;" ::"n"(ID), "r"(threads) : "memory");
+    tc::fence_after_sync();
+    return __all_sync(0xffffffffu, *good > n);
+}
+
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(bar)) : "memory");
+}
+
+// this warp's shared-memory operands (and TMEM reads) are done: one arrival for the warp
+__device__ __forceinline__ void warp_publish(uint64_t *bar, int lane)
 {
     tc::fence_smem_async();
     tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
 }
 
-// one (window, frame) pair of the tensor-core kernel, as one thread works it out ahead of time
-struct PairSetup {
-    int64_t q;              // the output index f * nwin + k
-    int p, k, f, gy, gx;    // pair, window, frame, gross offset
-    int sy, sx, mean;       // the chip's top-left corner and its rounded mean
-    float norm;
-    bool ok;                // the chip lies inside the frame and the reference window has texture
-};
+// the outputs of a pair without a peak, and of one whose peak is not refined, out of the kernel's way
+__device__ __noinline__ void tc_invalid(const CorrArgs *a, int64_t q)
+{
+    invalid_outputs(q, a->offset, a->peak, a->snr, a->cov);
+    if (a->peaks) a->peaks[q].valid = 0;
+}
+__device__ __noinline__ void tc_outputs(const CorrArgs *a, const float *fit, int u, int v, int gy, int gx, double sum, int count, int64_t q)
+{
+    peak_outputs(fit + 4, 3, a->M, u, v, a->R, gy, gx, a->W * a->W, sum, count, q, a->offset, a->peak, a->snr, a->cov);
+}
 
-
-// the rows of the variance-denominator box a TMA copy brings in: x rounded down to 4 floats
-// (16 bytes), so BW = M + 3 rounded up to 4 floats per row
-__host__ __device__ constexpr int tc_box_width(int M) { return (M + 3 + 3) / 4 * 4; }
-
-// dmap (global memory): the variance denominators of the group as a 3-D tensor (x = column,
-// y = row, z = frame), box tc_box_width(M) x M x 1
+// the chip of pair c into X by the gather warps (gw). rows16: a warp takes groups of 8 chip rows, lane
+// (r, c) = (lane & 7, lane >> 3) loads the aligned 16-byte chunks c, c + 4, c + 8 of row r (the chip's first
+// byte is byte o of chunk 0, the same o on every row), two steps ahead, and writes chip columns 16 q ..
+// 16 q + 15 (q = c + 4 k) from chunks q and q + 1 as two 16-byte FP16 pieces: the 8 lanes of one c fill
+// 128 contiguous bytes of a core matrix. Chunk q + 1 comes from its lane, not from memory again: lanes down
+// the rows cost the L1 a line's lookup each. Else a warp takes 8 rows x 4 pieces of 8 pixels as 4-byte
+// words (bytes where the rows are not word-aligned).
 template <int N>
-__global__ void __launch_bounds__(kTcThreads, 1) corr_tc_kernel(CorrArgs a, const uint4 *dtab, int *status,
-                                                                  const CUtensorMap *dmap)
+__device__ __forceinline__ void tc_gather(const CorrArgs &a, const PairSetup &c, unsigned char *X, bool rows16, int gw,
+                                          int lane)
+{
+    using G = TcGeo<N>;
+    const int L = a.L;
+    const __half2 off = __float2half2_rn(1024.0f + float(c.mean));
+    const uint8_t *chip = a.frames + c.f * a.fstride + int64_t(c.sy) * a.pitch + c.sx;
+    if (rows16) {
+        const int o = c.sx & 15, sw = o >> 2, sb = 8 * (o & 3);
+        const int r = lane & 7, cg = lane >> 3;
+        const int nq = (o + L + 15) >> 4;   // chunks holding chip bytes (they end inside the row)
+        const uint4 *rb = reinterpret_cast<const uint4 *>(chip - o);
+        const int pq = a.pitch >> 4;        // chunks per frame row
+        constexpr int NG = N / 8, NQ = N / 16, NK = (NQ + 4) / 4;    // groups, pieces, rounds of a row
+        auto load = [&](int g, int k) {
+            const int i = 8 * g + r, q = 4 * k + cg;
+            uint4 w = make_uint4(0u, 0u, 0u, 0u);
+            if (i < L && q < nq) w = ldg_here(rb + (i * pq + q));
+            return w;
+        };
+        auto next = [](int &g, int &k) {
+            if (++k == NK) {
+                k = 0;
+                g += kTcGather;
+            }
+        };
+        int g = gw, k = 0, g2 = gw, k2 = 0;   // this step, the step whose chunks are loaded
+        uint4 raw = load(g2, k2);
+        next(g2, k2);
+        uint4 then = load(g2, k2);
+        {
+#pragma unroll 1
+            for (; g < NG; next(g, k)) {
+                next(g2, k2);
+                const uint4 later = load(g2, k2);
+                // lane (r, 0) gives its next chunk to lane (r, 3), the others this one to their left
+                const bool give = cg == 0;
+                const int from = (lane + 8) & 31;
+                uint4 nx;
+                nx.x = __shfl_sync(0xffffffffu, give ? then.x : raw.x, from);
+                nx.y = __shfl_sync(0xffffffffu, give ? then.y : raw.y, from);
+                nx.z = __shfl_sync(0xffffffffu, give ? then.z : raw.z, from);
+                nx.w = __shfl_sync(0xffffffffu, give ? then.w : raw.w, from);
+                const int i = 8 * g + r, q = 4 * k + cg;
+                if (q < NQ) {
+                    // bytes 4 sw .. 4 sw + 19 of the 32 (sw is the same on every lane)
+                    const bool s2 = sw & 2, s1 = sw & 1;
+                    const uint32_t a0 = s2 ? raw.z : raw.x, a1 = s2 ? raw.w : raw.y, a2 = s2 ? nx.x : raw.z;
+                    const uint32_t a3 = s2 ? nx.y : raw.w, a4 = s2 ? nx.z : nx.x, a5 = s2 ? nx.w : nx.y;
+                    const uint32_t b[5] = {s1 ? a1 : a0, s1 ? a2 : a1, s1 ? a3 : a2, s1 ? a4 : a3, s1 ? a5 : a4};
+                    uint4 lo = make_uint4(0u, 0u, 0u, 0u), hi = make_uint4(0u, 0u, 0u, 0u);
+                    const int keep = i < L ? L - 16 * q : 0;   // chip columns from 16 q on
+                    if (keep > 0) {
+                        bytes_to_half(__funnelshift_r(b[0], b[1], sb), off, lo.x, lo.y);
+                        bytes_to_half(__funnelshift_r(b[1], b[2], sb), off, lo.z, lo.w);
+                        bytes_to_half(__funnelshift_r(b[2], b[3], sb), off, hi.x, hi.y);
+                        bytes_to_half(__funnelshift_r(b[3], b[4], sb), off, hi.z, hi.w);
+                    }
+                    if (keep < 16) {   // the 8 words of the 16 halves: zero past the chip
+                        uint32_t hv[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            if (2 * e >= keep) hv[e] = 0u;
+                            else if (2 * e + 1 >= keep) hv[e] &= 0xFFFFu;
+                        }
+                        lo = make_uint4(hv[0], hv[1], hv[2], hv[3]);
+                        hi = make_uint4(hv[4], hv[5], hv[6], hv[7]);
+                    }
+                    unsigned char *d = X + tc::k_major_offset(i, 16 * q, G::SBO_X, 128);
+                    *reinterpret_cast<uint4 *>(d) = lo;
+                    *reinterpret_cast<uint4 *>(d + 128) = hi;
+                }
+                raw = then;
+                then = later;
+            }
+        }
+        return;
+    }
+    const bool words = ((a.pitch | reinterpret_cast<uintptr_t>(a.frames) | int(a.fstride)) & 3) == 0;
+    constexpr int NCG = (N / 8 + 3) / 4;               // groups of 4 pieces per row
+    constexpr int NB = (N / 8) * NCG;                   // blocks of 8 rows x 4 pieces
+    constexpr int AHEAD = 2;                            // blocks loaded before they are used
+    for (int b0 = gw; b0 < NB; b0 += AHEAD * kTcGather) {
+        uint32_t w0[AHEAD], w1[AHEAD], w2[AHEAD];
+#pragma unroll
+        for (int t = 0; t < AHEAD; ++t) {
+            const int b = b0 + kTcGather * t;
+            const int i = 8 * (b / NCG) + (lane & 7), j0 = 8 * (4 * (b % NCG) + (lane >> 3));
+            w0[t] = w1[t] = w2[t] = 0u;
+            if (b < NB && i < L && j0 < L) {
+                const uint8_t *src = chip + int64_t(i) * a.pitch + j0;
+                const int left = L - j0;   // chip bytes from src on
+                if (words) {
+                    // the aligned words holding the chip bytes among src[0 .. 8)
+                    const uintptr_t addr = reinterpret_cast<uintptr_t>(src);
+                    const uint32_t *wp = reinterpret_cast<const uint32_t *>(addr & ~uintptr_t(3));
+                    const int sh = int(addr & 3);
+                    w0[t] = __ldg(wp);
+                    if (4 - sh < left) w1[t] = __ldg(wp + 1);
+                    if (sh > 0 && 8 - sh < left) w2[t] = __ldg(wp + 2);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        const uint32_t bt = e < left ? uint32_t(__ldg(src + e)) : 0u;
+                        if (e < 4) w0[t] |= bt << (8 * e);
+                        else w1[t] |= bt << (8 * (e - 4));
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < AHEAD; ++t) {
+            const int b = b0 + kTcGather * t;
+            const int i = 8 * (b / NCG) + (lane & 7), j0 = 8 * (4 * (b % NCG) + (lane >> 3));
+            if (b < NB && j0 < N) {
+                uint4 out = make_uint4(0u, 0u, 0u, 0u);
+                if (i < L && j0 < L) {
+                    uint32_t lo = w0[t], hi = w1[t];
+                    if (words) {
+                        const int sh = int(reinterpret_cast<uintptr_t>(chip + int64_t(i) * a.pitch + j0) & 3);
+                        lo = __funnelshift_r(w0[t], w1[t], 8 * sh);
+                        hi = __funnelshift_r(w1[t], w2[t], 8 * sh);
+                    }
+                    bytes_to_half(lo, off, out.x, out.y);
+                    bytes_to_half(hi, off, out.z, out.w);
+                    if (j0 + 8 > L) {   // the last piece of a row: zero past the chip
+                        const int keep = L - j0;   // 1 .. 7 pixels
+                        uint32_t hv[4] = {out.x, out.y, out.z, out.w};
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            if (2 * e >= keep) hv[e] = 0u;
+                            else if (2 * e + 1 >= keep) hv[e] &= 0xFFFFu;
+                        }
+                        out = make_uint4(hv[0], hv[1], hv[2], hv[3]);
+                    }
+                }
+                *reinterpret_cast<uint4 *>(X + tc::k_major_offset(i, j0, G::SBO_X, 128)) = out;
+            }
+        }
+    }
+}
+
+// the entry of the CTA's pair n, as soon as it is written; false if a role gave up
+__device__ __forceinline__ bool tc_entry(const PairSetup &e, uint32_t n, const volatile int *abort)
+{
+    bool ok = true;
+    while (*const_cast<const volatile uint32_t *>(&e.seq) != n + 1) {
+        if (*abort) {
+            ok = false;
+            break;
+        }
+        __nanosleep(64);
+    }
+    asm volatile("" ::: "memory");   // shared-memory reads stay in order
+    return __all_sync(__activemask(), ok);
+}
+
+template <int N>
+__global__ void __launch_bounds__(kTcThreads, 1) corr_tc_kernel(const __grid_constant__ CorrArgs a, const uint4 *dtab, int *status)
 {
     using G = TcGeo<N>;
     constexpr int NH = G::NH, KP = G::KP, NT = kTcThreads;
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ uint32_t tmem_base;
-    __shared__ __align__(8) uint64_t mbar, tbar;
-    __shared__ float s_best[NT / 32];
-    __shared__ int s_at[NT / 32];
-    __shared__ double s_sq[NT / 32];
+    __shared__ __align__(8) TcBars bar;
+    __shared__ __align__(8) uint64_t bar_last;
+    __shared__ int s_abort;
+    __shared__ PairSetup ring[4];      // the pairs in flight: gathered, drained, in the epilogue
+    __shared__ uint32_t s_good[5];     // the events the relay has told of (wake)
+    __shared__ uint32_t s_taken;       // the pairs whose epilogue's turn the gather warps have passed
+    __shared__ int s_key[kTcEpi], s_peak;   // the warps' largest values (as ints), the peak u M + v
+    __shared__ long long s_sq[kTcEpi];
+    __shared__ double s_wide;          // the part of the patch sum whose values do not fit the integers' range
     __shared__ float s_fit[9];
-    __shared__ int s_peak[3];   // the pending pair's peak: valid, u, v
-    __shared__ PairSetup s_next;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int quad = warp & 3, part = warp >> 2;
-    const int row = 32 * quad + lane;   // this thread's accumulator row (TMEM lane)
-    const bool compute = warp < kTcCompute, ctrl = tid == kTcCtrl;
-    unsigned char *A = smem, *X = smem + G::OFF_X;
-    float *dvs = reinterpret_cast<float *>(X);         // the variance denominators, from S2 on (X region)
-    const uint32_t sA = tc::smem_u32(A), sX = tc::smem_u32(X);
-    const uint32_t sDR = tc::smem_u32(smem + G::OFF_DR), sDI = tc::smem_u32(smem + G::OFF_DI);
+    constexpr int kRowWarps = (KP + 31) / 32;   // drain warps with rows, of each part
+    // the same on every lane, and known to be: the roles' branches are uniform
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const int quad = warp & 3;
+    const int row = 32 * quad + lane;   // the TMEM lane of an epilogue or drain thread
+    unsigned char *A = smem + G::OFF_A, *X = smem + G::OFF_X, *B5 = smem + G::OFF_B5;
+    volatile int *ab = &s_abort;
 
-    // the DFT matrices (already in the K-major layout), once per CTA
-    for (int i = tid; i < int(2 * G::D_BYTES / 16); i += NT)
-        reinterpret_cast<uint4 *>(smem + G::OFF_DR)[i] = __ldg(dtab + i);
+    // the DFT table (already in its layout), once per CTA
+    for (int i = tid; i < int(G::T_BYTES / 16); i += NT) reinterpret_cast<uint4 *>(smem)[i] = __ldg(dtab + i);
     if (warp == 0) tc::tmem_alloc(&tmem_base, G::TMEM_COLS);
-    if (ctrl) {
-        tc::mbar_init(&mbar, 1);
-        tc::mbar_init(&tbar, 1);
+    if (tid < 4) ring[tid].seq = 0;
+    if (tid == 0) {
+        s_abort = 0;
+        s_taken = 0;
+        for (int i = 0; i < 5; ++i) s_good[i] = 0;
+        s_peak = INT_MAX;
+        s_wide = 0.0;
+        tc::mbar_init(&bar.xfull, kTcGather);
+        tc::mbar_init(&bar.xfree, 1);
+        tc::mbar_init(&bar.stage[1], 1);
+        tc::mbar_init(&bar.stage[3], 1);
+        tc::mbar_init(&bar.afull, kTcDrain);
+        tc::mbar_init(&bar.stage[4], 1);
+        tc::mbar_init(&bar.pfull, kTcDrain);
+        tc::mbar_init(&bar.stage[0], 1);
+        tc::mbar_init(&bar.b5full, kTcDrain);
+        tc::mbar_init(&bar.stage[2], 1);
+        tc::mbar_init(&bar.cfree, kTcEpi);
+        tc::mbar_init(&bar_last, 1);
+        for (int i = 0; i < kTcSlots; ++i) {
+            tc::mbar_init(&bar.rfull[i], 1);
+            tc::mbar_init(&bar.rfree[i], kRowWarps);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    tc_publish();
-    const uint32_t tmem = tmem_base;
-    uint32_t tphase = 0;
-    const int BW = tc_box_width(a.M);
-    const uint32_t lane_base = uint32_t(32 * quad) << 16;
-    // the descriptors at k = 0 (built where they are used); the k-step s starts 256 s bytes on
-    // (16 s in the start-address field)
-#define B200_TC_DESCS                                                                                  \
-    const uint64_t dR0 = tc::smem_desc(sDR, 128, G::SBO_D), dI0 = tc::smem_desc(sDI, 128, G::SBO_D); \
-    const uint64_t a0A = tc::smem_desc(sA, 128, G::SBO_A), b0B5 = tc::smem_desc(sA, 128, G::SBO_B5);  \
-    (void)dR0; (void)dI0; (void)a0A; (void)b0B5;
-    uint32_t phase = 0;
-    const int L = a.L, M = a.M, R = a.R, W = a.W;
-    const int NO = (M + 15) / 16 * 16;
-    const int npairs = a.nwin * a.nf;
-    const size_t ss = size_t(a.w) + 1;
-    const bool words = ((a.pitch | reinterpret_cast<uintptr_t>(a.frames) | int(a.fstride)) & 3) == 0;
-
-    // the pair whose epilogue is pending: its S5 result in TMEM columns [C5, C5 + NO) while the next
-    // pair runs S1 .. S4; its variance denominators come by TMA into the X region after the next
-    // pair's S1, the normalization and argmax run during its S2, the SNR patch and the 3 x 3 fit
-    // values (read back from TMEM) during its S4, the FP64 peak solve during its S5
-    struct Prev {
-        int64_t q;
-        int f, sy, sx, gy, gx;
-        float scale;
-        bool live;
-    } prev{0, 0, 0, 0, 0, 0, 0.0f, false};
-    const uint32_t C5 = uint32_t(G::TMEM_COLS - NO);
-    float e_best = -2.0f;   // this thread's running argmax of the pending pair
-    int e_at = INT_MAX;
-    bool e_valid = false;   // the pending pair's surface has a positive peak
-    int e_pu = 0, e_pv = 0;
-
-    // the next pair's window, frame, position and chip mean, worked out by one thread of the last
-    // warp while the tensor cores run S1 (global-memory latency off the gather's path)
-    auto pair_setup = [&](int p) {
-        PairSetup o{};
-        o.p = p;
-        if (p >= npairs) return o;
-        o.k = p / a.nf;
-        o.f = p % a.nf;
-        o.q = int64_t(o.f) * a.nwin + o.k;
-        if (a.gross_mode == 1) {
-            o.gy = a.gross[2 * o.f];
-            o.gx = a.gross[2 * o.f + 1];
-        } else if (a.gross_mode == 2) {
-            o.gy = a.gross[2 * o.q];
-            o.gx = a.gross[2 * o.q + 1];
-        }
-        o.sy = a.down[o.k / a.nx] + o.gy - R;
-        o.sx = a.across[o.k % a.nx] + o.gx - R;
-        o.norm = a.norm[o.k];
-        o.ok = o.norm > 0 && o.sy >= 0 && o.sx >= 0 && o.sy + L <= a.h && o.sx + L <= a.w;
-        if (o.ok) {
-            const uint32_t *sat = a.sat + size_t(o.f) * a.sat_fstride;
-            const int sy = o.sy, sx = o.sx;
-            const uint32_t box = sat[(sy + L) * ss + sx + L] - sat[sy * ss + sx + L] - sat[(sy + L) * ss + sx] + sat[sy * ss + sx];
-            const uint32_t LL = uint32_t(L) * uint32_t(L);
-            o.mean = int((box + LL / 2) / LL);
-        }
-        return o;
-    };
-
-    // ---- X = chip - round(mean), FP16, K-major (rows i, columns j), zero outside L x L. Two ways:
-    // rows16 (frame rows on 16-byte boundaries and whole 16-byte chunks per row, the width a
-    // multiple of 16, so a row's chunks never leave it): aligned 16-byte chunk loads, below; else a
-    // warp takes 8 rows x 4 chunks of 8 pixels as 4-byte words, 32-byte pieces of 8 rows from global
-    // memory and one contiguous 512-byte store into shared memory. Every load of a thread first.
-    const bool rows16 = ((reinterpret_cast<uintptr_t>(a.frames) | uintptr_t(a.pitch) | uintptr_t(a.fstride)) & 15) == 0 &&
-                        (a.w & 15) == 0;
-    auto gather = [&](const PairSetup &c) {
-        if (!compute) return;
-        const __half2 off = __float2half2_rn(1024.0f + float(c.mean));
-        const uint8_t *chip = a.frames + c.f * a.fstride + int64_t(c.sy) * a.pitch + c.sx;
-        if (rows16 && N <= 160) {
-            // a warp takes groups of 8 chip rows: lane (r, c) = (lane & 7, lane >> 3) loads the aligned
-            // 16-byte chunks c, c + 4, c + 8 of row r (the chip's first byte is byte o of chunk 0, the
-            // same o on every row), then writes chip columns 16 q .. 16 q + 15 (q = c + 4 k) from
-            // chunks q and q + 1 as two 16-byte FP16 pieces: the 8 lanes of one c fill 128
-            // contiguous bytes of a core matrix
-            const int o = c.sx & 15, sw = o >> 2, sb = 8 * (o & 3);
-            const int r = lane & 7, cg = lane >> 3;
-            const int nq = (o + L + 15) >> 4;   // chunks holding chip bytes (they end inside the row)
-            const uint4 *rb = reinterpret_cast<const uint4 *>(chip - o);
-            const int64_t pq = a.pitch >> 4;    // chunks per frame row
-            constexpr int NK = ((N + 30) / 16 + 3) / 4;                  // rounds of 4 chunks (nq <= 4 NK)
-            constexpr int NG = N / 8;                                    // groups of 8 rows
-            constexpr int GPW = (NG + kTcCompute - 1) / kTcCompute;      // groups per warp
-            uint4 all[GPW][NK];   // every load of the warp first: one round trip to memory
-#pragma unroll
-            for (int t = 0; t < GPW; ++t) {
-                const int gi = warp + kTcCompute * t, i = 8 * gi + r;
-#pragma unroll
-                for (int k = 0; k < NK; ++k) {
-                    const int qq = cg + 4 * k;
-                    all[t][k] = make_uint4(0u, 0u, 0u, 0u);
-                    if (gi < NG && i < L && qq < nq) all[t][k] = __ldg(rb + int64_t(i) * pq + qq);
-                }
-            }
-#pragma unroll
-            for (int t = 0; t < GPW; ++t) {
-                const int gi = warp + kTcCompute * t, i = 8 * gi + r;
-                if (gi >= NG) break;   // warp-uniform
-                uint4 raw[NK + 1];
-#pragma unroll
-                for (int k = 0; k < NK; ++k) raw[k] = all[t][k];
-                raw[NK] = make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-                for (int k = 0; k < NK; ++k) {
-                    // chunk q + 1: lane (r, c + 1) of this round, or lane (r, 0) of the next
-                    const int down = (lane + 8) & 31;
-                    uint4 nx, nn;
-                    nx.x = __shfl_sync(0xffffffffu, raw[k].x, down);
-                    nx.y = __shfl_sync(0xffffffffu, raw[k].y, down);
-                    nx.z = __shfl_sync(0xffffffffu, raw[k].z, down);
-                    nx.w = __shfl_sync(0xffffffffu, raw[k].w, down);
-                    nn.x = __shfl_sync(0xffffffffu, raw[k + 1].x, r);
-                    nn.y = __shfl_sync(0xffffffffu, raw[k + 1].y, r);
-                    nn.z = __shfl_sync(0xffffffffu, raw[k + 1].z, r);
-                    nn.w = __shfl_sync(0xffffffffu, raw[k + 1].w, r);
-                    if (cg == 3) nx = nn;
-                    const int q = cg + 4 * k;
-                    if (q >= N / 16) continue;
-                    const uint32_t w[8] = {raw[k].x, raw[k].y, raw[k].z, raw[k].w, nx.x, nx.y, nx.z, nx.w};
-                    uint32_t b[5];   // bytes 4 sw .. 4 sw + 19 of the 32 (sw is the same on every lane)
-                    switch (sw) {
-                    case 0: b[0] = w[0]; b[1] = w[1]; b[2] = w[2]; b[3] = w[3]; b[4] = w[4]; break;
-                    case 1: b[0] = w[1]; b[1] = w[2]; b[2] = w[3]; b[3] = w[4]; b[4] = w[5]; break;
-                    case 2: b[0] = w[2]; b[1] = w[3]; b[2] = w[4]; b[3] = w[5]; b[4] = w[6]; break;
-                    default: b[0] = w[3]; b[1] = w[4]; b[2] = w[5]; b[3] = w[6]; b[4] = w[7]; break;
-                    }
-                    uint4 lo = make_uint4(0u, 0u, 0u, 0u), hi = make_uint4(0u, 0u, 0u, 0u);
-                    if (i < L) {
-                        bytes_to_half(__funnelshift_r(b[0], b[1], sb), off, lo.x, lo.y);
-                        bytes_to_half(__funnelshift_r(b[1], b[2], sb), off, lo.z, lo.w);
-                        bytes_to_half(__funnelshift_r(b[2], b[3], sb), off, hi.x, hi.y);
-                        bytes_to_half(__funnelshift_r(b[3], b[4], sb), off, hi.z, hi.w);
-                        const int keep = L - 16 * q;   // chip columns from 16 q on
-                        if (keep < 16) {   // the 8 words of the 16 halves: zero past the chip
-                            uint32_t hv[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-#pragma unroll
-                            for (int e = 0; e < 8; ++e) {
-                                if (2 * e >= keep) hv[e] = 0u;
-                                else if (2 * e + 1 >= keep) hv[e] &= 0xFFFFu;
-                            }
-                            lo = make_uint4(hv[0], hv[1], hv[2], hv[3]);
-                            hi = make_uint4(hv[4], hv[5], hv[6], hv[7]);
-                        }
-                    }
-                    *reinterpret_cast<uint4 *>(X + tc::k_major_offset(i, 16 * q, G::SBO_D, 128)) = lo;
-                    *reinterpret_cast<uint4 *>(X + tc::k_major_offset(i, 16 * q + 8, G::SBO_D, 128)) = hi;
-                }
-            }
-        } else {
-                constexpr int NCG = (N / 8 + 3) / 4;               // groups of 4 chunks per row
-                constexpr int NB = (N / 8) * NCG;                   // blocks of 8 rows x 4 chunks
-                constexpr int PERT = (NB + kTcCompute - 1) / kTcCompute;   // blocks per warp
-                constexpr int PERW = (PERT + 1) / 2;                    // in two rounds
-    #pragma unroll
-                for (int round = 0; round < 2; ++round) {
-                uint32_t w0[PERW], w1[PERW], w2[PERW];
-    #pragma unroll
-                for (int t = 0; t < PERW; ++t) {
-                    const int b = warp + kTcCompute * (t + round * PERW);
-                    const int i = 8 * (b / NCG) + (lane & 7), j0 = 8 * (4 * (b % NCG) + (lane >> 3));
-                    w0[t] = w1[t] = w2[t] = 0u;
-                    if (b < NB && t + round * PERW < PERT && i < L && j0 < L && j0 < N) {
-                        const uint8_t *src = chip + int64_t(i) * a.pitch + j0;
-                        const int left = L - j0;   // chip bytes from src on
-                        if (words) {
-                            // the aligned words holding the chip bytes among src[0 .. 8)
-                            const uintptr_t addr = reinterpret_cast<uintptr_t>(src);
-                            const uint32_t *wp = reinterpret_cast<const uint32_t *>(addr & ~uintptr_t(3));
-                            const int sh = int(addr & 3);
-                            w0[t] = __ldg(wp);
-                            if (4 - sh < left) w1[t] = __ldg(wp + 1);
-                            if (sh > 0 && 8 - sh < left) w2[t] = __ldg(wp + 2);
-                        } else {
-                            for (int e = 0; e < 8 && e < left; ++e) {
-                                const uint32_t bt = __ldg(src + e);
-                                if (e < 4) w0[t] |= bt << (8 * e);
-                                else w1[t] |= bt << (8 * (e - 4));
-                            }
-                        }
-                    }
-                }
-    #pragma unroll
-                for (int t = 0; t < PERW; ++t) {
-                    const int b = warp + kTcCompute * (t + round * PERW);
-                    const int i = 8 * (b / NCG) + (lane & 7), j0 = 8 * (4 * (b % NCG) + (lane >> 3));
-                    if (b < NB && t + round * PERW < PERT && j0 < N) {
-                        uint4 out = make_uint4(0u, 0u, 0u, 0u);
-                        if (i < L && j0 < L) {
-                            uint32_t lo = w0[t], hi = w1[t];
-                            if (words) {
-                                const int sh = int(reinterpret_cast<uintptr_t>(chip + int64_t(i) * a.pitch + j0) & 3);
-                                lo = __funnelshift_r(w0[t], w1[t], 8 * sh);
-                                hi = __funnelshift_r(w1[t], w2[t], 8 * sh);
-                            }
-                            bytes_to_half(lo, off, out.x, out.y);
-                            bytes_to_half(hi, off, out.z, out.w);
-                            if (j0 + 8 > L) {   // the last chunk of a row: zero past the chip
-                                const int keep = L - j0;   // 1 .. 7 pixels
-                                uint32_t *o = reinterpret_cast<uint32_t *>(&out);
-    #pragma unroll
-                                for (int e = 0; e < 4; ++e) {
-                                    if (2 * e >= keep) o[e] = 0u;
-                                    else if (2 * e + 1 >= keep) o[e] &= 0xFFFFu;
-                                }
-                            }
-                        }
-                        *reinterpret_cast<uint4 *>(X + tc::k_major_offset(i, j0, G::SBO_D, 128)) = out;
-                    }
-                }
-                }
-        }
-        tc::fence_smem_async();   // the chip is read by the tensor core
-    };
-
-    // ---- the pending pair's epilogue, in three parts (all threads call each)
-    // the denominator box (rows sy .. sy + M - 1, columns from sx rounded down to 4) into X
-    bool tma_pending = false;   // a denominator box is on its way (waited out before leaving)
-    auto epi_fetch = [&]() {
-        if (ctrl) {
-            tc::mbar_expect_tx(&tbar, uint32_t(BW * M * 4));
-            tc::tma_load_3d(dvs, dmap, prev.sx & ~3, prev.sy, prev.f, &tbar);
-        }
-        tma_pending = true;
-    };
-    // the normalized surface (thread v holds column v) and this thread's argmax; 16-column chunks
-    // of u alternate among the warps of a quadrant. false if the box did not arrive.
-    auto epi_normalize = [&]() -> bool {
-        const bool ok = tc::mbar_wait(&tbar, tphase);
-        tphase ^= 1u;
-        tma_pending = !ok;
-        e_best = -2.0f;
-        e_at = INT_MAX;
-        if (compute && 32 * quad < M) {
-            const int v = row;
-            const bool vin = v < M;
-            const float *__restrict__ dv = dvs + (prev.sx & 3) + v;
-            float *sv = a.surface ? a.surface + prev.q * M * M + v : nullptr;
-            for (int u0 = 16 * part; u0 < NO; u0 += 16 * kTcParts) {   // one 16-column chunk of u per TMEM wait
-                uint32_t cr[16];
-                tc::tmem_ld16_nowait(tmem + lane_base + C5 + uint32_t(u0), cr);
-                const int nu = M - u0 < 16 ? M - u0 : 16;   // rows u of the chunk inside the surface
-                float rho[16];
-#pragma unroll
-                for (int e = 0; e < 16; ++e) rho[e] = vin && e < nu ? dv[(u0 + e) * BW] : 0.0f;
-                tc::tmem_wait();
-#pragma unroll
-                for (int e = 0; e < 16; ++e) rho[e] *= __uint_as_float(cr[e]) * prev.scale;
-                if (vin) {
-                    if (sv) {
-#pragma unroll
-                        for (int e = 0; e < 16; ++e)
-                            if (e < nu) sv[(u0 + e) * M] = rho[e];
-                    }
-#pragma unroll
-                    for (int e = 0; e < 16; ++e)   // values <= -2 and NaN never win; ties keep the first u
-                        if (e < nu && rho[e] > e_best) {
-                            e_best = rho[e];
-                            e_at = u0 + e;
-                        }
-                }
-            }
-            e_at = e_at == INT_MAX ? INT_MAX : e_at * M + v;
-        }
-        return ok;
-    };
-    // the surface's argmax (the first in raster order if equal), then the SNR patch's sum of squares
-    // and the 3 x 3 fit's values, read back from TMEM with the same arithmetic
-    // (the compute warps only, with their own barrier: the control thread may still be issuing)
-    auto epi_peak = [&]() {
-        float best = e_best;
-        int at = e_at;
-        for (int o = 16; o > 0; o >>= 1) better(best, at, __shfl_xor_sync(0xffffffffu, best, o), __shfl_xor_sync(0xffffffffu, at, o));
-        if (lane == 0) {
-            s_best[warp] = best;
-            s_at[warp] = at;
-        }
-        asm volatile("bar.sync 1, %0;" ::"n"(32 * kTcCompute) : "memory");
-        best = lane < kTcCompute ? s_best[lane] : -2.0f;
-        at = lane < kTcCompute ? s_at[lane] : INT_MAX;
-        for (int o = 16; o > 0; o >>= 1) better(best, at, __shfl_xor_sync(0xffffffffu, best, o), __shfl_xor_sync(0xffffffffu, at, o));
-        e_valid = best > 0;
-        double sq = 0.0;
-        if (e_valid) {
-            e_pu = at / M;
-            e_pv = at % M;
-        }
-        if (tid == 0) {   // for the control thread's solve
-            s_peak[0] = e_valid;
-            s_peak[1] = e_pu;
-            s_peak[2] = e_pv;
-        }
-        if (e_valid) {
-            int i0, i1, j0, j1;
-            snr_patch(M, a.stat, e_pu, e_pv, i0, i1, j0, j1);
-            // the warps of a quadrant take alternate 16-row chunks of u from i0
-            if (compute && 32 * quad < j1 && 32 * quad + 32 > j0) {   // warp-uniform
-                for (int c0 = i0 + 16 * part; c0 < i1; c0 += 16 * kTcParts) {
-                    const int cb = c0 + 16 <= NO ? c0 : NO - 16;   // 16 columns inside [0, NO)
-                    uint32_t cr[16];
-                    tc::tmem_ld16_nowait(tmem + lane_base + C5 + uint32_t(cb), cr);
-                    tc::tmem_wait();
-                    const int v = row;
-                    if (v >= j0 && v < j1) {
-                        const float *__restrict__ dv = dvs + (prev.sx & 3) + v;
-#pragma unroll
-                        for (int e = 0; e < 16; ++e) {
-                            const int u = cb + e;
-                            if (u < c0 || u >= i1 || u >= c0 + 16) continue;
-                            float rho = dv[u * BW];
-                            rho *= __uint_as_float(cr[e]) * prev.scale;
-                            sq += double(rho) * double(rho);
-                            const int du = u - e_pu, dvv = v - e_pv;
-                            if (du >= -1 && du <= 1 && dvv >= -1 && dvv <= 1) s_fit[(du + 1) * 3 + dvv + 1] = rho;
-                        }
-                    }
-                }
-            }
-        }
-        for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-        if (lane == 0) s_sq[warp] = sq;
-    };
-    // the FP64 peak solve and the outputs (one thread), from s_fit and s_sq
-    auto epi_finish = [&]() {
-        e_valid = s_peak[0] != 0;
-        e_pu = s_peak[1];
-        e_pv = s_peak[2];
-        if (!e_valid) {
-            invalid_outputs(prev.q, a.offset, a.peak, a.snr, a.cov);
-            if (a.peaks) a.peaks[prev.q].valid = 0;
-            return;
-        }
-        int i0, i1, j0, j1;
-        snr_patch(M, a.stat, e_pu, e_pv, i0, i1, j0, j1);
-        double sum = 0.0;
-        for (int w = 0; w < kTcCompute; ++w) sum += s_sq[w];
-        if (a.peaks) {   // for the exact refinement of the peak, which writes the pair's outputs
-            PeakInfo &pi = a.peaks[prev.q];
-            pi.valid = 1;
-            pi.u = e_pu;
-            pi.v = e_pv;
-            pi.count = (i1 - i0) * (j1 - j0);
-            pi.sum = sum;
-            for (int t = 0; t < 9; ++t) pi.fit[t] = s_fit[t];
-            return;
-        }
-        peak_outputs(s_fit + 4, 3, M, e_pu, e_pv, R, prev.gy, prev.gx, W * W, sum, (i1 - i0) * (j1 - j0), prev.q,
-                     a.offset, a.peak, a.snr, a.cov);
-    };
-    // the whole epilogue of the pending pair, not overlapped (before a gather that needs X, and at
-    // the end); false if a wait gave up
-    auto epi_flush = [&]() -> bool {
-        if (!prev.live) return true;
-        epi_fetch();
-        const bool ok = epi_normalize();
-        if (compute) epi_peak();
-        __syncthreads();
-        if (ctrl) epi_finish();
-        prev.live = false;
-        return !__syncthreads_or(!ok);
-    };
-
-    if (ctrl) s_next = pair_setup(blockIdx.x);
-    __syncthreads();
-    PairSetup cur = s_next;
-    if (cur.p < npairs && cur.ok) gather(cur);
-    tc_publish();
-    bool failed = false;
-    while (cur.p < npairs) {
-        if (!cur.ok) {   // an invalid pair: its outputs now (the pending epilogue waits)
-            if (ctrl) {
-                invalid_outputs(cur.q, a.offset, a.peak, a.snr, a.cov);
-                if (a.peaks) a.peaks[cur.q].valid = 0;
-            }
-            if (a.surface)
-                for (int i = tid; i < M * M; i += NT) a.surface[cur.q * M * M + i] = 0.0f;
-            if (ctrl) s_next = pair_setup(cur.p + gridDim.x);
-            __syncthreads();
-            cur = s_next;
-            __syncthreads();
-            if (cur.p < npairs && cur.ok) {
-                if (!epi_flush()) {
-                    failed = true;
-                    break;
-                }
-                gather(cur);
-                tc_publish();
-            }
-            continue;
-        }
-        const int k = cur.k;
-        const float norm = cur.norm;
-
-        // ---- S1: Y = X [Dr | Di], tile t of 128 chip rows -> TMEM columns [2 KP t, 2 KP (t + 1))
-        if (ctrl) {
-            B200_TC_DESCS
-            const uint32_t id = tc::instr_desc(128, KP, false, false, false, false);
-#pragma unroll
-            for (int t = 0; t < G::T1; ++t) {
-                const uint64_t a0 = tc::smem_desc(sX + uint32_t(t * 16) * G::SBO_D, 128, G::SBO_D);
-#pragma unroll 2
-                for (int s = 0; s < N / 16; ++s) {
-                    tc::mma_f16(tmem + uint32_t(2 * KP * t), a0 + 16u * s, dR0 + 16u * s, id, s > 0);
-                    tc::mma_f16(tmem + uint32_t(2 * KP * t + KP), a0 + 16u * s, dI0 + 16u * s, id, s > 0);
-                }
-            }
-            tc::mma_commit(&mbar);
-        }
-        if (tid == kTcCtrl - 32) s_next = pair_setup(cur.p + gridDim.x);   // a compute warp, idle during S1
-        if (!tc_wait_all(&mbar, phase)) {
-            failed = true;
-            break;
-        }
-        // the pending pair's denominators into X (free: S1 has read the chip), under the S1 drain
-        if (prev.live) epi_fetch();
-        // S1 -> A2 (MN-major: m = kappa, k = part * N + i); the warps of a quadrant take the
-        // (Re or Im, column block) units in turn
-        for (int t = 0; t < G::T1; ++t) {
-            if (!compute || 128 * t + 32 * quad >= N) continue;   // warp-uniform
-            const int i = 128 * t + row;
-            constexpr int NC = KP % 32 ? 16 : 32;   // columns per wait
-            constexpr int NCH = KP / NC;
-            for (int un = part; un < 2 * NCH; un += kTcParts) {
-                const int ri = un / NCH, cb = NC * (un - ri * NCH);
-                float v[NC];
-                tc::tmem_ld_cols<NC>(tmem + lane_base + uint32_t(2 * KP * t + ri * KP + cb), v);
-                if (i < N) {
-#pragma unroll
-                    for (int c0 = 0; c0 < NC; c0 += 8)
-                        *reinterpret_cast<uint4 *>(A + tc::mn_major_offset(cb + c0, ri * N + i, G::SBO_A, 128)) = pack8(v + c0);
-                }
-            }
-        }
-        tc_publish();
-
-        // ---- S2: Z^T = Y^T D: Zr in TMEM columns [0, N), Zi in [N, 2N)
-        if (ctrl) {
-            B200_TC_DESCS
-            const uint32_t id = tc::instr_desc(128, N, true, false, false, false);
-            const uint32_t idn = tc::instr_desc(128, N, true, false, false, true);
-#pragma unroll 2
-            for (int s = 0; s < N / 16; ++s) {
-                const uint64_t ar = a0A + 16u * s, ai = a0A + uint32_t(N + 16 * s);   // Yr: k = i, Yi: k = N + i
-                tc::mma_f16(tmem, ar, dR0 + 16u * s, id, s > 0);        // Zr += Yr Dr
-                tc::mma_f16(tmem, ai, dI0 + 16u * s, idn, 1);           // Zr -= Yi Di
-                tc::mma_f16(tmem + N, ar, dI0 + 16u * s, id, s > 0);    // Zi += Yr Di
-                tc::mma_f16(tmem + N, ai, dR0 + 16u * s, id, 1);        // Zi += Yi Dr
-            }
-            tc::mma_commit(&mbar);
-        }
-        // the next pair's chip and reference spectrum into L2 while the tensor cores run S2 (its
-        // gather comes during this pair's S5, its S3 one pair later): a few prefetches per thread,
-        // every line holding bytes of the chip (inside the frame) or of the window's spectrum
-        if (compute) {
-            const PairSetup &nx = s_next;
-            if (nx.p < npairs && nx.ok) {
-                const uint8_t *chip = a.frames + nx.f * a.fstride + int64_t(nx.sy) * a.pitch + nx.sx;
-                for (int e = tid; e < 3 * L; e += 32 * kTcCompute) {   // a row of L <= 256 bytes spans <= 3 lines
-                    const int i = e / 3, l = e - 3 * i;
-                    const uintptr_t first = reinterpret_cast<uintptr_t>(chip + int64_t(i) * a.pitch);
-                    const uintptr_t line = (first & ~uintptr_t(127)) + 128 * uintptr_t(l);
-                    if (line <= first + uintptr_t(L - 1)) asm volatile("prefetch.global.L2 [%0];" ::"l"(line));
-                }
-                if (nx.k != k) {
-                    const char *r = reinterpret_cast<const char *>(a.spec_tc + size_t(nx.k) * (N / 2) * KP);
-                    constexpr int RL = (N / 2) * KP * 16 / 128;   // whole lines: KP is a multiple of 16
-                    for (int e = tid; e < RL; e += 32 * kTcCompute)
-                        asm volatile("prefetch.global.L2 [%0];" ::"l"(r + 128 * size_t(e)));
-                }
-            }
-        }
-        // this thread's row of the reference spectrum (S3): frequency pairs (ky, ky + 1) of the
-        // rows kappa side by side, KP float4 per pair (rows NH .. KP - 1 zero)
-        int eR = 0;
-        frexpf(float(W) * norm, &eR);   // W * norm < 2^eR, and max |R| <= W * norm
-        const int kap = row;
-        const float4 *rrow = a.spec_tc + size_t(k) * (N / 2) * KP + (kap < KP ? kap : 0);
-        const bool tma_ok = prev.live ? epi_normalize() : true;   // while the tensor cores run S2
-        if (!tc_wait_all(&mbar, phase, !tma_ok)) {
-            failed = true;
-            break;
-        }
-
-        // ---- S3: P = Z conj(R) 2^-(eR + 8) -> A4 (K-major: row kappa, k = part * N + ky); the
-        // 16-column chunks of ky alternate among the warps of a quadrant
-        if (compute && 32 * quad < KP) {
-            const float sc = ldexpf(1.0f, -(eR + 8));
-            for (int c0 = 16 * part; c0 < N; c0 += 16 * kTcParts) {
-                uint32_t zr[16], zi[16];
-                tc::tmem_ld16_nowait(tmem + lane_base + uint32_t(c0), zr);
-                tc::tmem_ld16_nowait(tmem + lane_base + uint32_t(N + c0), zi);
-                float4 rc[8];   // the spectrum's 16 frequencies of the chunk (the other warps of the quadrant hide the wait)
-#pragma unroll
-                for (int e = 0; e < 8; ++e) rc[e] = kap < KP ? __ldg(rrow + (c0 / 2 + e) * KP) : make_float4(0.f, 0.f, 0.f, 0.f);
-                tc::tmem_wait();
-                if (kap < KP) {
-#pragma unroll
-                    for (int hh = 0; hh < 2; ++hh) {   // 8 frequencies at a time
-                        float pr[8], pi[8];
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const float4 r = rc[4 * hh + e];
-                            const int z = 8 * hh + 2 * e;
-                            const float ar = __uint_as_float(zr[z]), ai = __uint_as_float(zi[z]);
-                            const float br = __uint_as_float(zr[z + 1]), bi = __uint_as_float(zi[z + 1]);
-                            pr[2 * e] = (ar * r.x + ai * r.y) * sc;
-                            pi[2 * e] = (ai * r.x - ar * r.y) * sc;
-                            pr[2 * e + 1] = (br * r.z + bi * r.w) * sc;
-                            pi[2 * e + 1] = (bi * r.z - br * r.w) * sc;
-                        }
-                        *reinterpret_cast<uint4 *>(A + tc::k_major_offset(kap, c0 + 8 * hh, G::SBO_A, 128)) = pack8(pr);
-                        *reinterpret_cast<uint4 *>(A + tc::k_major_offset(kap, N + c0 + 8 * hh, G::SBO_A, 128)) = pack8(pi);
-                    }
-                }
-            }
-        }
-        tc_publish();
-
-        // ---- S4: Q^T = P^T conj(D) for u < NO: Qr in TMEM columns [0, NO), Qi in [NO, 2 NO)
-        if (ctrl) {
-            B200_TC_DESCS
-            const uint32_t id = tc::instr_desc(128, NO, false, false, false, false);
-            const uint32_t idn = tc::instr_desc(128, NO, false, false, false, true);
-#pragma unroll 2
-            for (int s = 0; s < N / 16; ++s) {
-                const uint64_t ar = a0A + 16u * s, ai = a0A + uint32_t(N + 16 * s);   // Pr, Pi
-                tc::mma_f16(tmem, ar, dR0 + 16u * s, id, s > 0);                 // Qr += Pr Dr
-                tc::mma_f16(tmem, ai, dI0 + 16u * s, id, 1);                     // Qr += Pi Di
-                tc::mma_f16(tmem + uint32_t(NO), ar, dI0 + 16u * s, idn, s > 0); // Qi -= Pr Di
-                tc::mma_f16(tmem + uint32_t(NO), ai, dR0 + 16u * s, id, 1);      // Qi += Pi Dr
-            }
-            tc::mma_commit(&mbar);
-        }
-        if (prev.live && compute) epi_peak();   // while the tensor cores run S4
-        if (!tc_wait_all(&mbar, phase)) {
-            failed = true;
-            break;
-        }
-        // S4 -> B5 in the A region (MN-major: n = u, k = part * KP + kappa), with the Hermitian
-        // weights and 2^-9; the warps of a quadrant take the (Qr or Qi, 32-column block) units in turn
-        if (compute && 32 * quad < KP) {
-            const int kap = row;
-            const float wgt = kap >= NH ? 0.0f : ((kap == 0 || 2 * kap == N) ? 1.0f : 2.0f) * (1.0f / 512.0f);
-            const int nch = (NO + 31) / 32;
-            for (int un = part; un < 2 * nch; un += kTcParts) {
-                const int reim = un / nch, c0 = 32 * (un - reim * nch);
-                uint32_t r[32];
-                tc::tmem_ld16_nowait(tmem + lane_base + uint32_t(reim * NO + c0), r);
-                if (c0 + 16 < NO) tc::tmem_ld16_nowait(tmem + lane_base + uint32_t(reim * NO + c0 + 16), r + 16);
-                tc::tmem_wait();
-                if (kap < KP) {
-                    float v[32];
-#pragma unroll
-                    for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(r[e]);
-#pragma unroll
-                    for (int h = 0; h < 4; ++h)
-                        if (c0 + 8 * h < NO)
-                            *reinterpret_cast<uint4 *>(A + tc::mn_major_offset(c0 + 8 * h, reim * KP + kap, G::SBO_B5, 128)) =
-                                pack8(v + 8 * h, wgt);
-                }
-            }
-        }
-        tc_publish();
-
-        // ---- S5: c^T[v][u] = sum_kappa Dr[v][kappa] B5re[kappa][u] + Di[v][kappa] B5im[kappa][u], into
-        // TMEM columns [C5, C5 + NO), which no other stage writes: the epilogue reads it during the next pair
-        if (ctrl) {
-            B200_TC_DESCS
-            const uint32_t id = tc::instr_desc(128, NO, false, true, false, false);
-#pragma unroll 2
-            for (int s = 0; s < KP / 16; ++s) {
-                tc::mma_f16(tmem + C5, dR0 + 16u * s, b0B5 + 16u * s, id, s > 0);
-                tc::mma_f16(tmem + C5, dI0 + 16u * s, b0B5 + uint32_t(KP + 16 * s), id, 1);
-            }
-            tc::mma_commit(&mbar);
-        }
-        if (prev.live && ctrl) epi_finish();   // while the tensor cores run S5
-        const PairSetup next = s_next;
-        if (next.p < npairs && next.ok) gather(next);    // X is free: the pending epilogue is done
-        if (!tc_wait_all(&mbar, phase)) {
-            failed = true;
-            break;
-        }
-        prev = {cur.q, cur.f, cur.sy, cur.sx, cur.gy, cur.gx, ldexpf(1.0f, eR + 17) / (float(N) * float(N) * norm), true};
-        cur = next;
-    }
-    if (!failed && !epi_flush()) failed = true;
-    if (failed && ctrl && status) atomicExch(status, 3);
-    if (tma_pending) tc::mbar_wait(&tbar, tphase);   // no copy into this CTA's memory may outlive it
+    tc::fence_smem_async();
     tc::fence_before_sync();
     __syncthreads();
+    tc::fence_after_sync();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+    const uint32_t lane_base = uint32_t(32 * quad) << 16;
+    const int L = a.L, M = a.M, R = a.R, W = a.W;
+    const int NO = (M + 15) / 16 * 16;
+    // TMEM columns of Yr (then [P1|P3]), of Yi (then [P4|P2]); Q and c start at 0
+    const uint32_t CR = 2 * N, CI = uint32_t(NO);
+
+    if (warp == kTcControl) {
+        // ---- control: the MMAs, issued by one thread of the warp
+        const uint32_t one = tc::elect_one();
+        const uint32_t sT = tc::smem_u32(smem), sA = tc::smem_u32(A), sX = tc::smem_u32(X), sB5 = tc::smem_u32(B5);
+        // the table's rows along M or N, contraction over its columns (k-step s: + KT s) ...
+        const uint64_t c_rows = tc::smem_desc(sT, G::SBO_T, 128);
+        // ... and its columns along M, contraction over its rows (k-step s: + 16 s); S starts N/2 rows on
+        const uint64_t c_cols = tc::smem_desc(sT, 128, G::SBO_T);
+        const uint64_t dX = tc::smem_desc(sX, 128, G::SBO_X), dA = tc::smem_desc(sA, 128, G::SBO_A);
+        const uint64_t dB5 = tc::smem_desc(sB5, 128, G::SBO_B5);
+        constexpr uint32_t KT = 2u * uint32_t(G::RT);
+        const uint32_t idn = tc::instr_desc(128, N, false, false, false, false);
+        const uint32_t id5 = tc::instr_desc(128, NO, true, true, false, false);
+        auto wait = [&](uint64_t *b, uint32_t par) { return tc_wait_warp(b, par, ab); };
+        // one pair per turn: the back of pair n - 1 (S4, S5) woven into the front of pair n (S1, S2), as
+        // eight runs of MMAs through one loop
+        bool ok = true, end = false;
+        for (uint32_t n = 0; ok && !end; ++n) {
+            const uint32_t par = n & 1u, prv = par ^ 1u;
+#pragma unroll 1
+            for (int step = n ? 0 : 2; step < 8 && ok; ++step) {
+                if (step == 3 && !n) step = 5;        // no pair before
+                if (step == 5 && end) break;
+                uint32_t d = 0, acc = 0;                 // columns d: A from da (and, S5, B from db)
+                uint64_t da = dA, db = dB5, *done = nullptr;
+                if (step == 0) {          // S4: c of pair n - 2 is read (its columns are Q's), and S2's products (theirs too)
+                    ok = (n < 2 || wait(&bar.cfree, par)) && wait(&bar.pfull, prv);
+                } else if (step == 1) {
+                    d = N;
+                    da += N;
+                    done = &bar.stage[0];
+                } else if (step == 2) {   // S1, Yr
+                    ok = wait(&bar.xfull, par);
+                    end = ok && __any_sync(0xffffffffu, ring[n & 3].end);
+                    d = CR;
+                    da = c_rows;
+                    done = &bar.stage[1];
+                } else if (step == 3) {   // S5, C then S
+                    ok = wait(&bar.b5full, prv);
+                    da = c_cols;
+                } else if (step == 4) {
+                    da = c_cols + N / 2;
+                    db += KP;
+                    acc = 1;
+                    done = &bar.stage[2];
+                } else if (step == 5) {   // S1, Yi
+                    d = CI;
+                    da = c_rows + N / 2;
+                    done = &bar.stage[3];
+                } else if (step == 6) {   // S2
+                    ok = wait(&bar.afull, par);
+                    d = CR;
+                } else {
+                    d = CI;
+                    da += N;
+                    done = &bar.stage[4];
+                }
+                if (!ok) break;
+                // (unrolled by kind, the steps constant: 55 cycles an MMA to issue)
+                if (step == 3 || step == 4) {
+#pragma unroll
+                    for (int s = 0; s < KP / 16; ++s) tc::mma_f16_warp(tmem, da + 16u * s, db + 16u * s, id5, s ? 1u : acc, one);
+                } else if (step == 2 || step == 5) {
+                    if (!end)
+#pragma unroll
+                        for (int s = 0; s < N / 16; ++s) tc::mma_f16_warp(tmem + d, da + KT * s, dX + 16u * s, idn, s > 0, one);
+                } else {
+#pragma unroll
+                    for (int s = 0; s < N / 16; ++s) tc::mma_f16_warp(tmem + d, da + 16u * s, c_rows + KT * s, idn, s > 0, one);
+                }
+                if (done && one) {
+                    if (step == 2 && end) mbar_arrive(done);   // no pair: the drain warps leave
+                    else tc::mma_commit(done);
+                    if (step == 5) tc::mma_commit(&bar.xfree);
+                }
+            }
+        }
+        if (!ok) *ab = 1;
+    } else if (warp == kTcRelay) {
+        // ---- relay: the MMAs complete in the order they are issued in. After a wait gives up, the turn's
+        // wake-ups (and the epilogue's next) go on without waiting, uncounted, and who is woken leaves.
+        constexpr int DW = 32 * (kTcDrain + 1), EW = 32 * (kTcEpi + 1);
+        bool ok = true, end = false;
+        for (uint32_t n = 0; ok && !end; ++n) {
+            int told = 0;   // C of the pair before: 1 come about, 2 not
+#pragma unroll 1
+            for (int ev = n ? 0 : 1; ev < 5; ++ev) {   // Q, Yr, C, Yi, Z: Q and C of the pair before
+                if (ev == 2 && !n) continue;
+                const uint32_t m = ev == 0 || ev == 2 ? n - 1 : n;
+                ok = ok && tc_wait_warp(&bar.stage[ev], m & 1u, ab);
+                if (ev == 1) end = ok && __any_sync(0xffffffffu, ring[n & 3].end);
+                wake(kTcWake + ev, ev == 2 ? EW : DW, &s_good[ev], m, ok, lane);
+                if (ev == 2) told = ok ? 1 : 2;
+                if (end && ev == (n ? 2 : 1)) break;
+            }
+            if (!ok && told < 2) wake(kTcWakeC, EW, &s_good[2], told || !n ? n : n - 1, false, lane);
+        }
+    } else if (warp == kTcSetup) {
+        // ---- the pairs ahead: lane l works out the CTA's next pair but l, then they are published in
+        // order, each when its entry of the ring is free; invalid pairs are written here and passed over
+        const int npairs = a.nwin * a.nf;
+        const size_t ss = size_t(a.w) + 1;
+        uint32_t n = 0;
+        bool ok = true;
+        auto publish = [&](PairSetup &c, bool mine) -> bool {   // entry n, by the lane whose it is
+            while (n >= 4 && *const_cast<volatile uint32_t *>(&s_taken) < n - 3) {
+                if (*ab) return false;
+                __nanosleep(100);
+            }
+            __threadfence_block();
+            if (mine) {
+                c.seq = n;   // not a pair's yet
+                ring[n & 3] = c;
+                __threadfence_block();
+                *const_cast<volatile uint32_t *>(&ring[n & 3].seq) = n + 1;
+            }
+            ++n;
+            return true;
+        };
+        for (int p0 = blockIdx.x; p0 < npairs && ok; p0 += 32 * gridDim.x) {
+            const int p = p0 + lane * gridDim.x;
+            PairSetup c{};
+            bool valid = false;
+            if (p < npairs) {
+                c.k = p / a.nf;
+                c.f = p % a.nf;
+                c.q = int64_t(c.f) * a.nwin + c.k;
+                if (a.gross_mode == 1) {
+                    c.gy = a.gross[2 * c.f];
+                    c.gx = a.gross[2 * c.f + 1];
+                } else if (a.gross_mode == 2) {
+                    c.gy = a.gross[2 * c.q];
+                    c.gx = a.gross[2 * c.q + 1];
+                }
+                c.sy = a.down[c.k / a.nx] + c.gy - R;
+                c.sx = a.across[c.k % a.nx] + c.gx - R;
+                const float norm = a.norm[c.k];
+                valid = norm > 0 && c.sy >= 0 && c.sx >= 0 && c.sy + L <= a.h && c.sx + L <= a.w;
+                if (valid) {
+                    const uint32_t *sat = a.sat + size_t(c.f) * a.sat_fstride;
+                    const size_t t0 = c.sy * ss + c.sx, t1 = t0 + L * ss;
+                    const uint32_t box = sat[t1 + L] - sat[t0 + L] - sat[t1] + sat[t0];
+                    const uint32_t LL = uint32_t(L) * uint32_t(L);
+                    c.mean = int((box + LL / 2) / LL);
+                    int eR = 0;
+                    frexpf(float(W) * norm, &eR);   // the reference spectrum is scaled by 2^-(eR + 8)
+                    c.scale = ldexpf(1.0f, eR + 17) / (float(N) * float(N) * norm);
+                } else {
+                    tc_invalid(&a, c.q);
+                }
+            }
+            const uint32_t todo = __ballot_sync(0xffffffffu, valid), bad = __ballot_sync(0xffffffffu, p < npairs && !valid);
+            if (a.surface)
+                for (uint32_t b = bad; b; b &= b - 1) {
+                    const int64_t q = __shfl_sync(0xffffffffu, c.q, __ffs(int(b)) - 1);
+                    for (int i = lane; i < M * M; i += 32) a.surface[q * M * M + i] = 0.0f;
+                }
+            for (uint32_t b = todo; b && ok; b &= b - 1) {
+                const int src = __ffs(int(b)) - 1;
+                ok = __all_sync(0xffffffffu, publish(c, lane == src));
+                // the window's spectrum into L2 before its pairs (on the CTAs around, at the same time) want it,
+                // by one of them
+                const int k = __shfl_sync(0xffffffffu, c.k, src), f = __shfl_sync(0xffffffffu, c.f, src);
+                const char *r = reinterpret_cast<const char *>(a.spec_tc + size_t(k) * (N / 2) * KP);
+                if (f == 0)
+#pragma unroll 1
+                    for (int i = lane; i < (N / 2) * KP * 16 / 128; i += 32)
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(r + 128 * size_t(i)));
+            }
+        }
+        PairSetup c{};
+        c.end = true;
+        if (ok) publish(c, lane == 0);
+    } else if (warp == kTcFetch) {
+        // ---- the reference spectrum of the pairs, chunk after chunk
+        if (lane == 0) {
+            uint32_t g = 0;   // chunks so far: slot g % 4, its use g / 4
+            for (uint32_t n = 0;; ++n) {
+                const PairSetup &e = ring[n & 3];
+                if (!tc_entry(e, n, ab) || e.end) break;
+                const float4 *r = a.spec_tc + size_t(e.k) * (N / 2) * KP;
+                if (n && !tc_wait(&bar.stage[2], (n - 1) & 1u, ab)) break;   // S5 has read what the ring overwrites
+                bool ok = true;
+#pragma unroll 1
+                for (int j = 0; j < G::NR; ++j, ++g) {
+                    const uint32_t slot = g % kTcSlots, use = g / kTcSlots;
+                    if (use && !(ok = tc_wait(&bar.rfree[slot], (use - 1) & 1u, ab))) break;
+                    tc::mbar_expect_tx(&bar.rfull[slot], G::R_BYTES);
+                    tc::bulk_load(B5 + slot * G::R_BYTES, r + size_t(8 * j) * KP, G::R_BYTES, &bar.rfull[slot]);
+                }
+                if (!ok) break;
+            }
+            // no copy into this CTA's memory may outlive it
+            int none = 0;
+            for (uint32_t u = g > kTcSlots ? g - kTcSlots : 0; u < g; ++u)
+                tc_wait(&bar.rfull[u % kTcSlots], (u / kTcSlots) & 1u, &none);
+        }
+    } else if (warp < 16 && quad < 3) {
+        // ---- drain: thread kappa holds row kappa of every stage's accumulator
+        const int part = warp >> 2;   // of the quadrant's four warps
+        const int kap = row;
+        const bool has = 32 * quad < KP, in = kap < KP;   // rows of this warp (warp-uniform), of this thread
+        constexpr int DW = 32 * (kTcDrain + 1);
+        const uint32_t tl = tmem + lane_base;
+        const float wgt = kap >= NH ? 0.0f : ((kap == 0 || 2 * kap == N) ? 1.0f : 2.0f) * (1.0f / 512.0f);
+        for (uint32_t n = 0;; ++n) {
+            // S1 -> S2's operand (row kappa, k = (Re | Im) N + i), 16 columns at a time
+            auto drain1 = [&](uint32_t col, int im) {
+                if (!has) return;
+#pragma unroll 1
+                for (int c = 16 * part; c < N; c += 16 * kTcParts) {
+                    float y[16];
+                    tc::tmem_ld_cols<16>(tl + col + uint32_t(c), y);
+                    if (im && kap == 0) {   // the Nyquist row is not S's row 0
+#pragma unroll
+                        for (int t = 0; t < 16; ++t) y[t] = 0.0f;
+                    }
+                    if (in) {
+                        unsigned char *o = A + tc::k_major_offset(kap, im * N + c, G::SBO_A, 128);
+                        *reinterpret_cast<uint4 *>(o) = pack8(y);
+                        *reinterpret_cast<uint4 *>(o + 128) = pack8(y + 8);
+                    }
+                }
+            };
+            if (!woken<kTcWakeYr>(DW, &s_good[1], n)) break;
+            if (__any_sync(0xffffffffu, ring[n & 3].end)) break;
+            drain1(CR, 0);
+            if (!woken<kTcWakeYi>(DW, &s_good[3], n)) break;
+            drain1(CI, 1);
+            warp_publish(&bar.afull, lane);
+
+            // S3: chunk t, dealt to the quadrant's warps, gives P at ky = r, r = 8 t .. 8 t + 7, and at
+            // N - r, r = 8 t + 1 .. 8 t + 8 (whole 16-byte pieces of the operand both), two frequencies per
+            // instruction. R's ring holds them in pairs: (x, x', y, y') of two ky, then of their mirrors.
+            if (!woken<kTcWakeZ>(DW, &s_good[4], n)) break;
+#pragma unroll 1
+            for (int t = part; t < G::NR && has; t += kTcParts) {
+                const uint32_t g = n * uint32_t(G::NR) + uint32_t(t), slot = g % kTcSlots;
+                tc_wait_warp(&bar.rfull[slot], (g / kTcSlots) & 1u, ab);   // if it gives up, the next wake-up says so
+                const ulonglong2 *rs = reinterpret_cast<const ulonglong2 *>(B5 + slot * G::R_BYTES) + (in ? kap : 0);
+                uint32_t o1[4], o2[4], o3[4], o4[4];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    // columns r of the four products, and columns r + 1 for the mirrors
+                    uint32_t a[4][4], m[4][4];
+                    const uint32_t z = tl + uint32_t(8 * t + 4 * h);
+                    tc::tmem_ld4_nowait(z + CR, a[0]);
+                    tc::tmem_ld4_nowait(z + CI + N / 2, a[1]);
+                    tc::tmem_ld4_nowait(z + CR + N / 2, a[2]);
+                    tc::tmem_ld4_nowait(z + CI, a[3]);
+                    tc::tmem_ld4_nowait(z + CR + 1, m[0]);
+                    tc::tmem_ld4_nowait(z + CI + N / 2 + 1, m[1]);
+                    tc::tmem_ld4_nowait(z + CR + N / 2 + 1, m[2]);
+                    tc::tmem_ld4_nowait(z + CI + 1, m[3]);
+                    tc::tmem_wait();
+                    // column 0 of P2 and P3 is ky = N/2: column N/2 of P1 and P4, which lie before them
+                    if (h == 0 && t == 0) a[1][0] = a[2][0] = 0u;
+                    if (h == 1 && t == G::NR - 1) m[1][3] = m[2][3] = 0u;
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const ulonglong2 rd = rs[(4 * h + 2 * j) * KP], rm = rs[(4 * h + 2 * j + 1) * KP];
+                        const f32x2 a1 = pair2(a[0], j), a2 = pair2(a[1], j), m1 = pair2(m[0], j), m3 = pair2(m[2], j);
+                        const f32x2 ar = sub2(a1, a2), na = sub2(a2, a1), ai = add2(pair2(a[2], j), pair2(a[3], j));
+                        const f32x2 br = add2(m1, pair2(m[1], j)), bi = sub2(pair2(m[3], j), m3), nb = neg2(br);
+                        o1[2 * h + j] = half2_bits(fma2(ar, rd.x, mul2(ai, rd.y)));
+                        o2[2 * h + j] = half2_bits(fma2(ai, rd.x, mul2(na, rd.y)));
+                        o3[3 - 2 * h - j] = half2_swapped(fma2(br, rm.x, mul2(bi, rm.y)));
+                        o4[3 - 2 * h - j] = half2_swapped(fma2(bi, rm.x, mul2(nb, rm.y)));
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bar.rfree[slot]);
+                if (in) {
+                    unsigned char *o = A + tc::k_major_offset(kap, 8 * t, G::SBO_A, 128);
+                    unsigned char *m = A + tc::k_major_offset(kap, N - 8 * t - 8, G::SBO_A, 128);
+                    *reinterpret_cast<uint4 *>(o) = make_uint4(o1[0], o1[1], o1[2], o1[3]);
+                    *reinterpret_cast<uint4 *>(o + 16 * N) = make_uint4(o2[0], o2[1], o2[2], o2[3]);
+                    *reinterpret_cast<uint4 *>(m) = make_uint4(o3[0], o3[1], o3[2], o3[3]);
+                    *reinterpret_cast<uint4 *>(m + 16 * N) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
+                }
+            }
+            warp_publish(&bar.pfull, lane);
+
+            // S4 -> S5's operand (MN-major: n = u, k = (Re | Im) KP + kappa) with the Hermitian weights and
+            // 2^-9: chunk t gives u = 8 t .. 8 t + 7, and N - u for 8 t + 1 .. 8 t + 8 where the surface
+            // reaches
+            if (!woken<kTcWakeQ>(DW, &s_good[0], n)) break;
+            const f32x2 wr = both(wgt), wi = both(kap == 0 ? 0.0f : wgt);   // S5 reads the Nyquist row as S's row 0
+            auto load = [&](int u, uint32_t (&q)[4][8]) {   // Pr C, Pi S, Pi C, Pr S
+                tc::tmem_ld8_nowait(tl + uint32_t(u), q[0]);
+                tc::tmem_ld8_nowait(tl + uint32_t(3 * N / 2 + u), q[1]);
+                tc::tmem_ld8_nowait(tl + uint32_t(N + u), q[2]);
+                tc::tmem_ld8_nowait(tl + uint32_t(N / 2 + u), q[3]);
+                tc::tmem_wait();
+            };
+            auto put = [&](int u, const uint32_t (&r)[4], const uint32_t (&m)[4]) {
+                if (!in) return;
+                unsigned char *o = B5 + tc::mn_major_offset(u, kap, G::SBO_B5, 128);
+                *reinterpret_cast<uint4 *>(o) = make_uint4(r[0], r[1], r[2], r[3]);
+                *reinterpret_cast<uint4 *>(o + 16 * KP) = make_uint4(m[0], m[1], m[2], m[3]);
+            };
+#pragma unroll 1
+            for (int t = part; t < G::NR && has; t += kTcParts) {
+                uint32_t q[4][8], r[4], m[4];
+                if (8 * t < M) {
+                    load(8 * t, q);
+                    if (t == 0) q[1][0] = q[3][0] = 0u;   // column 0 of the S products is u = N/2
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        r[j] = half2_bits(mul2(add2(pair2(q[0], j), pair2(q[1], j)), wr));
+                        m[j] = half2_bits(mul2(sub2(pair2(q[2], j), pair2(q[3], j)), wi));
+                    }
+                    put(8 * t, r, m);
+                }
+                if (N - 8 * t - 8 < M) {
+                    load(8 * t + 1, q);
+                    if (t == G::NR - 1) q[1][7] = q[3][7] = 0u;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        r[3 - j] = half2_swapped(mul2(sub2(pair2(q[0], j), pair2(q[1], j)), wr));
+                        m[3 - j] = half2_swapped(mul2(add2(pair2(q[2], j), pair2(q[3], j)), wi));
+                    }
+                    put(N - 8 * t - 8, r, m);
+                }
+            }
+            warp_publish(&bar.b5full, lane);
+        }
+    } else if (warp < 24) {
+        // ---- epilogue: thread v holds column v of the surface, the two warps of a quadrant alternate
+        // groups of 8 rows u
+        const int ew = warp - 16, part = ew >> 2, v = row, dw = a.dpitch;
+        const bool mine = 32 * quad < M, vin = v < M;   // of this warp, of this thread
+        for (uint32_t n = 0;; ++n) {
+            const PairSetup &e = ring[n & 3];
+            const bool known = tc_entry(e, n, ab);      // if not, the wake-up says to leave
+            if (known && __any_sync(0xffffffffu, e.end)) break;
+            const float *dcol = a.dinv + (vin ? v : 0);
+            if (known) dcol += size_t(e.f) * a.dinv_fstride + size_t(e.sy) * dw + e.sx;
+            const float scale = e.scale;
+            // 8 rows' denominators (rows past the surface lie in the table or its padding, unused); the first
+            // 24 are on their way while the tensor core works on the pair
+            auto fetch = [&](float (&d)[8], int u0) {
+                if (!mine || !known || u0 >= M) return;
+                const float *p = dcol + u0 * dw;
+#pragma unroll
+                for (int t = 0; t < 8; ++t, p += dw) d[t] = ldg_here(p);
+            };
+            auto rows = [&](int u0, float (&x)[8]) {   // denominators to surface
+                uint32_t cr[8];
+                tc::tmem_ld8_nowait(tmem + lane_base + uint32_t(u0), cr);
+                tc::tmem_wait();
+#pragma unroll
+                for (int t = 0; t < 8; ++t) x[t] *= __uint_as_float(cr[t]) * scale;
+            };
+            float d0[8], d1[8], d2[8];
+            fetch(d0, 8 * part);
+            fetch(d1, 8 * part + 16);
+            fetch(d2, 8 * part + 32);
+            if (!woken<kTcWakeC>(32 * (kTcEpi + 1), &s_good[2], n)) break;
+            // this thread's largest value and its row (NaN never wins, ties keep the first)
+            float best = -2.0f;
+            int bu = 0;
+            if (mine) {
+#pragma unroll 1
+                for (int u0 = 8 * part; u0 < M; u0 += 16) {
+                    rows(u0, d0);
+                    if (a.surface && vin) {
+                        float *sv = a.surface + (e.q * M + u0) * M + v;
+#pragma unroll
+                        for (int t = 0; t < 8; ++t)
+                            if (u0 + t < M) sv[t * M] = d0[t];
+                    }
+                    float m = -2.0f;
+                    int first = 0;
+#pragma unroll
+                    for (int t = 7; t >= 0; --t) {
+                        const bool up = d0[t] >= m && u0 + t < M;
+                        m = up ? d0[t] : m;
+                        first = up ? u0 + t : first;
+                    }
+                    bu = m > best ? first : bu;
+                    best = m > best ? m : best;
+#pragma unroll
+                    for (int t = 0; t < 8; ++t) {
+                        d0[t] = d1[t];
+                        d1[t] = d2[t];
+                    }
+                    fetch(d2, u0 + 48);
+                }
+            }
+            // positive floats order as their bits do; a surface without a positive value has no peak
+            const int mykey = __reduce_max_sync(0xffffffffu, vin ? __float_as_int(best) : INT_MIN);
+            if (lane == 0) s_key[ew] = mykey;
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * kTcEpi) : "memory");
+            const int key = __reduce_max_sync(0xffffffffu, s_key[lane & 7]);
+            const bool valid = key > 0;
+            if (valid && mykey == key) {   // warp-uniform: where, the first in raster order if equal
+                const int at = __reduce_min_sync(0xffffffffu, vin && __float_as_int(best) == key ? bu * M + v : INT_MAX);
+                if (lane == 0) atomicMin(&s_peak, at);
+            }
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * kTcEpi) : "memory");
+            const int at = valid ? s_peak : 0, pu = at / M, pv = at - pu * M;
+            int i0 = 0, i1 = 0, j0 = 0, j1 = 0;
+            // the SNR patch's sum of squares and the 3 x 3 values, with the same arithmetic. The values are
+            // summed as integers, rounded to 2^-sh with sh as large as the patch's count allows (26 at 21 x
+            // 21: below FP32's own rounding of a value above 1/8), each product and the sum exact.
+            long long sq = 0;
+            int sh = 0;
+            auto release = [&] {   // this warp reads c's columns no more
+                tc::fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bar.cfree);
+            };
+            if (valid) {
+                snr_patch(M, a.stat, pu, pv, i0, i1, j0, j1);
+                sh = (29 + __clz((i1 - i0) * (j1 - j0))) >> 1;   // count 4 2^(2 sh) < 2^63
+            }
+            // the warp's first group with a row of the patch, if it holds columns of it (warp-uniform)
+            const bool cols = valid && 32 * quad < j1 && 32 * quad + 32 > j0;
+            int u0 = 8 * part + (max(i0 - 7 - 8 * part, 0) + 15) / 16 * 16;
+            if (!cols || u0 >= i1) {
+                release();
+            } else {
+                const float up = __int_as_float((127 + sh) << 23);
+                const bool col = v >= j0 && v < j1;
+                const uint32_t fv = uint32_t(v - pv + 1);
+#pragma unroll 1
+                for (; u0 < i1; u0 += 32) {   // two groups at a time
+                    fetch(d0, u0);
+                    fetch(d1, u0 + 16);
+                    rows(u0, d0);
+                    if (u0 + 16 < M) rows(u0 + 16, d1);
+                    if (u0 + 32 >= i1) release();
+#pragma unroll 1
+                    for (int ub = u0; ub < u0 + 32; ub += 16) {
+                        bool wide = false;
+#pragma unroll
+                        for (int t = 0; t < 8; ++t) {
+                            const uint32_t fu = uint32_t(ub + t - pu + 1);
+                            float x = d0[t];
+                            if (fu < 3u && fv < 3u) s_fit[fu * 3 + fv] = x;
+                            if (!col || ub + t < i0 || ub + t >= i1) x = 0.0f;
+                            const int z = __float2int_rn(x * up);
+                            sq += (long long)z * z;
+                            wide |= !(fabsf(x) < 2.0f);
+                            d0[t] = x;
+                        }
+                        if (__any_sync(0xffffffffu, wide)) {   // values of 2 and more, or none: in FP64
+#pragma unroll
+                            for (int t = 0; t < 8; ++t) {
+                                const int z = __float2int_rn(d0[t] * up);
+                                sq -= (long long)z * z;
+                                if (d0[t] != 0.0f) atomicAdd(&s_wide, double(d0[t]) * double(d0[t]));
+                            }
+                        }
+#pragma unroll
+                        for (int t = 0; t < 8; ++t) d0[t] = d1[t];
+                    }
+                }
+                for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+            }
+            if (lane == 0) s_sq[ew] = sq;
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * kTcEpi) : "memory");
+            if (ew == 0 && lane == 0) {
+                const int64_t q = e.q;
+                const int gy = e.gy, gx = e.gx;
+                *const_cast<volatile uint32_t *>(&s_taken) = n + 1;   // nobody reads the entry any more
+                s_peak = INT_MAX;
+                if (!valid) {
+                    tc_invalid(&a, q);
+                } else {
+                    long long total = 0;
+#pragma unroll 1
+                    for (int w = 0; w < kTcEpi; ++w) total += s_sq[w];
+                    const double sum = double(total) * __hiloint2double((1023 - 2 * sh) << 20, 0) + s_wide;
+                    s_wide = 0.0;
+                    const int count = (i1 - i0) * (j1 - j0);
+                    if (a.peaks) {   // for the exact refinement of the peak, which writes the pair's outputs
+                        PeakInfo &pi = a.peaks[q];
+                        pi.valid = 1;
+                        pi.u = pu;
+                        pi.v = pv;
+                        pi.count = count;
+                        pi.sum = sum;
+                        for (int t = 0; t < 9; ++t) pi.fit[t] = s_fit[t];
+                    } else {
+                        tc_outputs(&a, s_fit, pu, pv, gy, gx, sum, count, q);
+                    }
+                }
+            }
+        }
+    } else {
+        // ---- gather: the chip of the next pair, S1's operand (K-major rows i, columns j, zero outside L x L)
+        // aligned 16-byte chunks when the frame rows start on 16-byte boundaries and hold whole chunks
+        const bool rows16 = ((reinterpret_cast<uintptr_t>(a.frames) | uintptr_t(a.pitch) | uintptr_t(a.fstride)) & 15) == 0 &&
+                            (a.w & 15) == 0;
+        for (uint32_t n = 0;; ++n) {
+            const PairSetup &c = ring[n & 3];
+            if (!tc_entry(c, n, ab)) break;
+            // S1 of the pair before has read X
+            if (n && !tc_wait_warp(&bar.xfree, (n - 1) & 1u, ab)) break;
+            const bool end = __any_sync(0xffffffffu, c.end);
+            if (!end) tc_gather<N>(a, c, X, rows16, warp - 24, lane);
+            warp_publish(&bar.xfull, lane);
+            if (end) break;
+        }
+    }
+    // every role has left its loop; after a wait gave up, what was issued is waited out (with the same
+    // bound) before the tensor memory goes back
+    __syncthreads();
+    if (s_abort && warp == kTcControl) {
+        if (tc::elect_one()) tc::mma_commit(&bar_last);
+        int none = 0;
+        tc_wait(&bar_last, 0, &none);
+        if (status && lane == 0) atomicExch(status, 3);
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
     if (warp == 0) tc::tmem_dealloc(tmem, G::TMEM_COLS);
-#undef B200_TC_DESCS
 }
 
-// the reference spectra in the order S3 of the tensor-core form reads them: for window k and the
-// frequency pair (ky, ky + 1) = (2 p, 2 p + 1), the rows kappa < KP side by side, one float4
-// (R[kappa][2 p], R[kappa][2 p + 1]) each, rows NH .. KP - 1 zero. spec holds nwin x NH x N.
-__global__ void spec_tc_kernel(const float2 *__restrict__ spec, float4 *__restrict__ out, int N, int nwin)
+// the reference spectra as S3 of the tensor-core form reads them: for window k and chunk t of 8
+// frequencies, the rows kappa < KP side by side, 8 float4 each: for the pairs j, j + 1 (j = 0, 2, 4, 6)
+// (x, x', y, y') of R[kappa][8 t + j], R[kappa][8 t + j + 1], then of R[kappa][N - 8 t - 1 - j] and
+// R[kappa][N - 8 t - 2 - j]; scaled by 2^-(e + 8), 2^e > W norm (exact); rows NH .. KP - 1 zero. spec
+// holds nwin x NH x N.
+__global__ void spec_tc_kernel(const float2 *__restrict__ spec, const float *__restrict__ norm, int W, float4 *__restrict__ out,
+                               int N, int nwin)
 {
     const int NH = N / 2 + 1, KP = tc_kp(N);
     const int64_t total = int64_t(nwin) * (N / 2) * KP;
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += int64_t(gridDim.x) * blockDim.x) {
         const int kap = int(i % KP);
-        const int64_t kp = i / KP;
-        const int pr = int(kp % (N / 2));
-        const int64_t k = kp / (N / 2);
+        const int64_t ks = i / KP;
+        const int slot = int(ks % (N / 2)), t = slot / 8, j = slot & 6;
+        const int64_t k = ks / (N / 2);
         float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
         if (kap < NH) {
-            const float2 *r = spec + (k * NH + kap) * N + 2 * pr;
-            o = make_float4(r[0].x, r[0].y, r[1].x, r[1].y);
+            int eR = 0;
+            frexpf(float(W) * norm[k], &eR);
+            const float sc = ldexpf(1.0f, -(eR + 8));
+            const float2 *row = spec + (k * NH + kap) * N;
+            const bool mirror = slot & 1;
+            const float2 x = row[mirror ? N - 8 * t - 1 - j : 8 * t + j], y = row[mirror ? N - 8 * t - 2 - j : 8 * t + j + 1];
+            o = make_float4(x.x * sc, y.x * sc, x.y * sc, y.y * sc);
         }
         out[i] = o;
     }
@@ -793,8 +1059,8 @@ __global__ void spec_tc_kernel(const float2 *__restrict__ spec, float4 *__restri
 
 #endif   // __CUDACC__
 
-// the DFT matrices of the tensor-core form as the kernel keeps them in shared memory: Dr then Di,
-// each K-major (rows r, columns c, both in [0, N)), FP16 bits; out holds 2 * N * N halves
+// the DFT table of the tensor-core form as the kernel keeps it in shared memory (tc_table_offset), FP16
+// bits; out holds tc_rt(N) * N halves
 void tc_dft_table(int N, uint16_t *out);
 
 }   // namespace b200

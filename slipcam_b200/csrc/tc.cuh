@@ -83,6 +83,29 @@ __device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64
         "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate));
 }
 
+// The same by a whole warp, one of whose threads (`leader`, from elect_one) issues it. In a branch that
+// every thread of the warp takes, the compiler keeps the descriptors in uniform registers, which is where
+// the instruction wants them: 39 cycles from one MMA to the next at most, against 90 when a single thread
+// runs the loop and each operand is moved there first (measured; an M = 128, N = 80 MMA itself takes 52).
+__device__ __forceinline__ void mma_f16_warp(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                             uint32_t accumulate, uint32_t leader)
+{
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader));
+}
+
+// 1 in one thread of the (converged) warp, 0 in the others
+__device__ __forceinline__ uint32_t elect_one()
+{
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.b32 %0, 1, 0, q;\n\t}" : "=r"(e));
+    return e;
+}
+
 // the mbarrier arrives when every MMA issued so far by this thread has completed
 __device__ __forceinline__ void mma_commit(uint64_t *mbar)
 {
@@ -155,6 +178,21 @@ __device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, uint32_t *r)
         : "r"(taddr));
 }
 
+// 4 and 8 columns, without waiting
+__device__ __forceinline__ void tmem_ld4_nowait(uint32_t taddr, uint32_t (&r)[4])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr));
+}
+
+__device__ __forceinline__ void tmem_ld8_nowait(uint32_t taddr, uint32_t (&r)[8])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+}
+
 __device__ __forceinline__ void tmem_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // NC (a multiple of 16) consecutive columns of this thread's lane into v, one wait for all
@@ -177,15 +215,14 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *mbar, uint32_t bytes)
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(mbar)), "r"(bytes) : "memory");
 }
 
-// a 3-D box of a tensor map into shared memory (TMA, no multicast); completion is counted on mbar.
-// The innermost coordinate x times the element size must be a multiple of 16 bytes.
-__device__ __forceinline__ void tma_load_3d(void *dst, const void *tmap, int x, int y, int z, uint64_t *mbar)
+// `bytes` (a multiple of 16, both addresses 16-byte aligned) global -> shared by the copy engine; completion
+// is counted on mbar
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *mbar)
 {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
-            smem_u32(dst)),
-        "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(smem_u32(mbar))
-        : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(smem_u32(mbar))
+                 : "memory");
 }
 
 // 4-byte asynchronous copies global -> shared, completed by cp_async_wait_all
