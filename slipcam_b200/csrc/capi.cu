@@ -42,7 +42,8 @@ using namespace b200;
 
 namespace {
 
-constexpr int kThreads = 256;   // threads per correlation CTA
+constexpr int kThreads = 256;   // threads per CTA of the reference spectra
+constexpr int kBigThreads = 512;   // of the big transform's correlation: 3.31 ms against 3.89 with 256, 3.58 with 448 (3,712 pairs)
 thread_local std::string g_create_error;
 
 struct Failure {
@@ -249,7 +250,7 @@ void prepare()
     int dev = 0;
     CK(cudaGetDevice(&dev));
     if (dev >= 0 && dev < 64 && done[dev]) return;
-    CK(cudaFuncSetAttribute(corr_kernel<N, kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Geo<N>::smem_bytes)));
+    CK(cudaFuncSetAttribute(corr_kernel<N, corr_threads(N)>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Geo<N>::smem_bytes)));
     CK(cudaFuncSetAttribute(spectra_kernel<N, kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Geo<N>::smem_bytes)));
     if (dev >= 0 && dev < 64) done[dev] = true;
 }
@@ -258,7 +259,7 @@ template <int N>
 void launch_corr(const CorrArgs &a, cudaStream_t s)
 {
     prepare<N>();
-    corr_kernel<N, kThreads><<<unsigned(a.nwin) * a.nf, kThreads, Geo<N>::smem_bytes, s>>>(a);
+    corr_kernel<N, corr_threads(N)><<<unsigned(a.nwin) * a.nf, corr_threads(N), Geo<N>::smem_bytes, s>>>(a);
 }
 
 // threads per pair of the latency-bound correlation (one frame of a chain at a time)
@@ -299,7 +300,7 @@ void prepare_big()
     CK(cudaGetDevice(&dev));
     if (dev >= 0 && dev < 64 && done[dev]) return;
     const int smem = int(BigGeo<kBigN>::smem_bytes);
-    CK(cudaFuncSetAttribute(corr_big_cluster_kernel<kBigN, kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    CK(cudaFuncSetAttribute(corr_big_cluster_kernel<kBigN, kBigThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             int(BigClusterGeo<kBigN>::smem_bytes)));
     CK(cudaFuncSetAttribute(spectra_big_kernel<kBigN, kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     if (dev >= 0 && dev < 64) done[dev] = true;
@@ -314,10 +315,10 @@ int big_clusters()
     if (dev >= 0 && dev < 64 && cached[dev]) return cached[dev];
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(unsigned(num_sms() / 2 * 2), 1, 1);
-    cfg.blockDim = dim3(kThreads, 1, 1);
+    cfg.blockDim = dim3(kBigThreads, 1, 1);
     cfg.dynamicSmemBytes = BigClusterGeo<kBigN>::smem_bytes;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, corr_big_cluster_kernel<kBigN, kThreads>, &cfg) != cudaSuccess || n < 1) {
+    if (cudaOccupancyMaxActiveClusters(&n, corr_big_cluster_kernel<kBigN, kBigThreads>, &cfg) != cudaSuccess || n < 1) {
         cudaGetLastError();
         n = num_sms() / 2;
     }
@@ -331,7 +332,7 @@ void launch_corr_big(const CorrArgs &a, float2 *, cudaStream_t s)
 {
     prepare_big();
     const int clusters = std::min(a.nwin * a.nf, big_clusters());
-    corr_big_cluster_kernel<kBigN, kThreads><<<unsigned(2 * clusters), kThreads, BigClusterGeo<kBigN>::smem_bytes, s>>>(a);
+    corr_big_cluster_kernel<kBigN, kBigThreads><<<unsigned(2 * clusters), kBigThreads, BigClusterGeo<kBigN>::smem_bytes, s>>>(a);
 }
 
 template <int N>
@@ -698,9 +699,6 @@ struct b200_handle {
             B200_DISPATCH_TC(N, launch_corr_tc, a, dt, d_status.p, s);
         } else if (N == kBigN) {
             launch_corr_big(a, d_big.p, s);
-        } else if (N == 192) {
-            // one 154 KB tile per SM: 512 threads per pair keep 16 warps resident instead of 8
-            launch_corr_latency<192>(a, s);
         } else {
             B200_DISPATCH(N, launch_corr, a, s);
         }

@@ -351,6 +351,7 @@ __device__ void corr_big_cluster_pair(const CorrArgs &a, int p, int rank, float2
 template <int N, int NT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NT, 1) corr_big_cluster_kernel(CorrArgs a)
 {
+    static_assert(NT % 32 == 0, "whole warps");
     namespace cg = cooperative_groups;
     using C = BigClusterGeo<N>;
     cg::cluster_group cluster = cg::this_cluster();

@@ -238,6 +238,7 @@ __global__ void __launch_bounds__(NT) spectra_kernel(SpectraArgs a)
 template <int N, int NT>
 __device__ __forceinline__ void corr_pair(const CorrArgs &a, int k, int f, float2 *S)
 {
+    static_assert(NT % 32 == 0, "whole warps: the shuffles and the per-warp sums count on it");
     using G = Geo<N>;
     float2 *TW = S + size_t(N) * G::NHP, *TWI = TW + N;
     float *Sr = reinterpret_cast<float *>(S);
@@ -327,10 +328,20 @@ __device__ __forceinline__ void corr_pair(const CorrArgs &a, int k, int f, float
     surface_peak<NT>(Sr, G::RP, M, R, a.stat, gy, gx, a.W * a.W, q, a.offset, a.peak, a.snr, a.cov, nullptr);
 }
 
+// Threads per pair and pairs an SM holds at once, by transform size. The passes hand a row pair or two
+// columns to a warp, so few warps per pair leave none of them idle in the last round, and the registers
+// of a pair's threads bound how many pairs run side by side; the shared tile does from N = 128 on. Measured
+// (kernel, against 256 threads and two pairs at every size): N = 64 (window 32, search 16, 10,368 pairs)
+// 0.395 ms against 0.536, 256 threads x 4 pairs 0.410; N = 96 0.451 against 0.611, 256 x 3 0.480; N = 128
+// 1.85 (256 x 3) against 192 x 4 2.03; N = 160 2.62 against 2.82, 384 2.88, 352 2.99, 512 3.47; N = 192 one
+// pair, 640 threads 10.8 against 512 11.8, 576 12.0, 704 13.8. Multiples of 32 only.
+constexpr int corr_threads(int N) { return N <= 96 ? 128 : N <= 128 ? 256 : N <= 160 ? 320 : 640; }
+constexpr int corr_blocks(int N) { return N <= 64 ? 8 : N <= 96 ? 5 : N <= 128 ? 3 : N <= 160 ? 2 : 1; }
+
 // the correlation of one (window, frame) pair per CTA; blockIdx.x = window * nf + frame, so the
 // CTAs of one window (one reference spectrum) run together and share it through L2
 template <int N, int NT>
-__global__ void __launch_bounds__(NT, (N <= 160 ? 2 : 1)) corr_kernel(CorrArgs a)
+__global__ void __launch_bounds__(NT, corr_blocks(N)) corr_kernel(CorrArgs a)
 {
     extern __shared__ float4 smem_raw[];
     corr_pair<N, NT>(a, blockIdx.x / a.nf, blockIdx.x % a.nf, reinterpret_cast<float2 *>(smem_raw));
