@@ -120,7 +120,7 @@ struct HostBuf {
 struct Slot {
     DevBuf<uint8_t> frames;
     DevBuf<uint32_t> sat;
-    DevBuf<int64_t> sat2;
+    DevBuf<uint32_t> sat2;
     DevBuf<float> dinv;
     DevBuf<int2> bstat;         // {box sum, dinv} beside dinv (the exact tensor-core form, the refinement)
     DevBuf<PeakInfo> peaks;     // the tensor-core kernel's peaks, for their exact refinement
@@ -439,12 +439,23 @@ void launch_spectra(const SpectraArgs &a, int nwin, cudaStream_t s)
     default: fail(B200_EINVAL, "no kernel for the FFT size " + std::to_string(N_));               \
     }
 
+// T2 = uint32_t: the tables of the correlation; int64_t: the exact table of squares
+template <class T2>
 void launch_sat(const uint8_t *frames, int64_t fstride, int pitch, int nf, int h, int w, uint32_t *sat,
-                int64_t *sat2, cudaStream_t s)
+                T2 *sat2, cudaStream_t s)
 {
     const int64_t sfs = int64_t(h + 1) * (w + 1);
     sat_rows_kernel<<<dim3(unsigned((h + 7) / 8), unsigned(nf)), 256, 0, s>>>(frames, fstride, pitch, h, w, sat, sat2, sfs);
-    sat_cols_kernel<<<dim3(unsigned((w + 1 + 31) / 32), unsigned(nf)), dim3(32, 8), 0, s>>>(h, w, sat, sat2, sfs);
+    sat_cols_kernel<<<dim3(unsigned((w + 1 + 31) / 32), unsigned(nf)), dim3(32, kSatSegs), 0, s>>>(h, w, sat, sat2, sfs);
+}
+
+// the variance denominators of nf frames' W x W boxes from their tables
+void launch_dinv(const uint32_t *sat, const uint32_t *sat2, int nf, int h, int w, int W, float *dinv, int64_t dfs, int dpitch,
+                 int2 *bstat, cudaStream_t s)
+{
+    constexpr int per = 128 * kDinvCols;
+    dinv_kernel<<<dim3(unsigned((w - W + per) / per), unsigned(h - W + 1), unsigned(nf)), 128, 0, s>>>(
+        sat, sat2, int64_t(h + 1) * (w + 1), h, w, W, dinv, dfs, dpitch, bstat);
 }
 
 }   // namespace
@@ -473,12 +484,12 @@ struct b200_handle {
     DevBuf<PeakInfo> d_peaks;    // device-path peaks of the tensor-core form
     DevBuf<int> d_queue;         // and the refinement's queue
     DevBuf<uint32_t> d_sat;      // device-path scratch
-    DevBuf<int64_t> d_sat2;
+    DevBuf<uint32_t> d_sat2;
     DevBuf<float> d_dinv;
     Slot slot[2];
     bool slots_ready = false;    // the slots are allocated (ensure_slots)
     DevBuf<uint32_t> d_csat;     // coarse tracking: two sets of tables of kCoarseGroup frames
-    DevBuf<int64_t> d_csat2;
+    DevBuf<uint32_t> d_csat2;
     DevBuf<float> d_cdinv;
     DevBuf<uint16_t> d_dtab;     // the FP16 DFT matrices of the tensor-core form
     DevBuf<int> d_status;        // device status word (3: a tensor-core wait gave up)
@@ -575,7 +586,7 @@ struct b200_handle {
     // the tables and the correlation of nf frames (device memory) on stream s; bstat (the box table
     // beside dinv) serves the exact tensor-core form
     void run_group(const uint8_t *frames, int pitch, int nf, const int32_t *gross, int gross_mode,
-                   uint32_t *sat, int64_t *sat2, float *dinv, int2 *bstat, PeakInfo *peaks, int *queue, float *offset,
+                   uint32_t *sat, uint32_t *sat2, float *dinv, int2 *bstat, PeakInfo *peaks, int *queue, float *offset,
                    float *peak, float *snr, float *cov, float *surface, cudaStream_t s, bool tables_done = false)
     {
         const int arith = group_arith(bstat);
@@ -624,13 +635,12 @@ struct b200_handle {
     }
 
     // the summed-area tables and the variance denominators of nf frames (and the box table)
-    void run_tables(const uint8_t *frames, int pitch, int nf, uint32_t *sat, int64_t *sat2, float *dinv, cudaStream_t s,
+    void run_tables(const uint8_t *frames, int pitch, int nf, uint32_t *sat, uint32_t *sat2, float *dinv, cudaStream_t s,
                     int2 *bstat = nullptr)
     {
         const int64_t fstride = int64_t(pitch) * height;
         launch_sat(frames, fstride, pitch, nf, height, width, sat, sat2, s);
-        dinv_kernel<<<dim3(unsigned((width - W + 1 + 127) / 128), unsigned(height - W + 1), unsigned(nf)), 128, 0, s>>>(
-            sat, sat2, sat_size(), height, width, W, dinv, dinv_size(), dpitch(), bstat);
+        launch_dinv(sat, sat2, nf, height, width, W, dinv, dinv_size(), dpitch(), bstat, s);
     }
 
     // the correlation of nf frames with their tables at sat / dinv, in the form `arith`
@@ -1180,7 +1190,7 @@ int b200_correlate_device_noalloc(b200_handle *h, const uint8_t *frames, int n, 
         if (n == 0) return;
         if (!frames || pitch < h->width || !offset || !peak || !snr || !cov)
             fail(B200_EINVAL, "null input or output, or a pitch below the width");
-        // the tables of one frame: 32-bit and 64-bit summed-area tables, variance denominators
+        // the room for one frame: two summed-area tables (8 bytes an entry for the squares), variance denominators
         const size_t b32 = size_t(h->sat_size()) * sizeof(uint32_t), b64 = size_t(h->sat_size()) * sizeof(int64_t);
         const size_t bd = size_t(h->dinv_size()) * sizeof(float);
         const size_t per_frame = align256(b32) + align256(b64) + align256(bd);
@@ -1203,7 +1213,7 @@ int b200_correlate_device_noalloc(b200_handle *h, const uint8_t *frames, int n, 
         const int G = int(std::min<size_t>(kNoAllocBytes / per_frame, size_t(h->group)));
         unsigned char *q = static_cast<unsigned char *>(base);
         uint32_t *sat = reinterpret_cast<uint32_t *>(q);
-        int64_t *sat2 = reinterpret_cast<int64_t *>(q + align256(G * b32));
+        uint32_t *sat2 = reinterpret_cast<uint32_t *>(q + align256(G * b32));
         float *dinv = reinterpret_cast<float *>(q + align256(G * b32) + align256(G * b64));
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         const int nwin = h->nwin;
@@ -1212,8 +1222,7 @@ int b200_correlate_device_noalloc(b200_handle *h, const uint8_t *frames, int n, 
             const int nf = std::min(G, n - f0);
             const size_t q0 = size_t(f0) * nwin;
             launch_sat(frames + f0 * fstride, fstride, pitch, nf, h->height, h->width, sat, sat2, s);
-            dinv_kernel<<<dim3(unsigned((h->width - h->W + 1 + 127) / 128), unsigned(h->height - h->W + 1), unsigned(nf)),
-                          128, 0, s>>>(sat, sat2, h->sat_size(), h->height, h->width, h->W, dinv, h->dinv_size(), h->dpitch());
+            launch_dinv(sat, sat2, nf, h->height, h->width, h->W, dinv, h->dinv_size(), h->dpitch(), nullptr, s);
             CorrArgs a{};
             a.frames = frames + f0 * fstride;
             a.fstride = fstride;
@@ -1558,7 +1567,7 @@ int b200_coarse_track_device(b200_handle *h, const uint8_t *frames, int n, int p
             h->d_cdinv.alloc(2 * size_t(G) * h->dinv_size());
         }
         uint32_t *sat[2] = {h->d_csat.p, h->d_csat.p + size_t(G) * h->sat_size()};
-        int64_t *sat2[2] = {h->d_csat2.p, h->d_csat2.p + size_t(G) * h->sat_size()};
+        uint32_t *sat2[2] = {h->d_csat2.p, h->d_csat2.p + size_t(G) * h->sat_size()};
         float *dinv[2] = {h->d_cdinv.p, h->d_cdinv.p + size_t(G) * h->dinv_size()};
         cudaEvent_t *ready = h->coarse_ev, *consumed = h->coarse_ev + 2, start = h->coarse_ev[4];
         cudaStream_t side = h->copy;
@@ -1810,7 +1819,7 @@ struct b200_group {
     cudaEvent_t ev_in = nullptr, ev_out = nullptr;
     int cap = 0;                         // frames the per-call tables hold
     DevBuf<uint32_t> sat;
-    DevBuf<int64_t> sat2;
+    DevBuf<uint32_t> sat2;
     std::vector<int> wsizes;             // the distinct window sizes, one denominator table each
     std::vector<DevBuf<float>> dinv;
     DevBuf<int> counter;
@@ -1923,8 +1932,7 @@ struct b200_group {
         launch_sat(frames, int64_t(pitch) * height, pitch, n, height, width, sat.p, sat2.p, stream);
         for (size_t wi = 0; wi < wsizes.size(); ++wi) {
             const int W = wsizes[wi];
-            dinv_kernel<<<dim3(unsigned((width - W + 1 + 127) / 128), unsigned(height - W + 1), unsigned(n)), 128, 0, stream>>>(
-                sat.p, sat2.p, sat_size(), height, width, W, dinv[wi].p, dinv_size(), dpitch());
+            launch_dinv(sat.p, sat2.p, n, height, width, W, dinv[wi].p, dinv_size(), dpitch(), nullptr, stream);
         }
         if (per_grid) {
             for (int i = 0; i < host_args.ngrids; ++i) {
