@@ -1,6 +1,7 @@
 // diff.cu -- the launches of the differentiable correlation (diff.cuh): one CTA per pair for
 // every stage; the FFT stages are instantiated for the FFT sizes of the correlation kernels.
 
+#include <algorithm>
 #include <stdexcept>
 #include <string>
 
@@ -8,8 +9,6 @@
 
 namespace b200 {
 namespace {
-
-constexpr int kNT = 256;
 
 void ck(cudaError_t e, const char *what)
 {
@@ -24,9 +23,9 @@ void prepare()
     int dev = 0;
     ck(cudaGetDevice(&dev), "cudaGetDevice");
     if (dev >= 0 && dev < 64 && done[dev]) return;
-    ck(cudaFuncSetAttribute(diff_corr_kernel<N, kNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Geo<N>::smem_bytes)),
+    ck(cudaFuncSetAttribute(diff_corr_kernel<N, corr_threads(N)>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Geo<N>::smem_bytes)),
        "cudaFuncSetAttribute");
-    ck(cudaFuncSetAttribute(adjoint_kernel<N, kNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Geo<N>::smem_bytes)),
+    ck(cudaFuncSetAttribute(adjoint_kernel<N, corr_threads(N)>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Geo<N>::smem_bytes)),
        "cudaFuncSetAttribute");
     ck(cudaFuncSetAttribute(diff_stats_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 256 * kStatStrip * 8),
        "cudaFuncSetAttribute");
@@ -37,14 +36,14 @@ template <int N>
 void corr(const DiffArgs &a, unsigned pairs, cudaStream_t s)
 {
     prepare<N>();
-    diff_corr_kernel<N, kNT><<<pairs, kNT, Geo<N>::smem_bytes, s>>>(a);
+    diff_corr_kernel<N, corr_threads(N)><<<pairs, corr_threads(N), Geo<N>::smem_bytes, s>>>(a);
 }
 
 template <int N>
 void adjoint(const DiffArgs &a, unsigned pairs, cudaStream_t s)
 {
     prepare<N>();
-    adjoint_kernel<N, kNT><<<pairs, kNT, Geo<N>::smem_bytes, s>>>(a);
+    adjoint_kernel<N, corr_threads(N)><<<pairs, corr_threads(N), Geo<N>::smem_bytes, s>>>(a);
 }
 
 #define B200_DIFF_DISPATCH(N_, F, ...)                                                             \
@@ -77,7 +76,7 @@ void launch_diff_forward(const DiffArgs &a, int N, cudaStream_t s)
     const unsigned pairs = pair_grid(a);
     if (!pairs) return;
     B200_DIFF_DISPATCH(N, prepare);
-    diff_gather_kernel<<<pairs, 256, 0, s>>>(a);
+    diff_gather_kernel<<<pairs, 256, size_t(kStripRows) * a.L * sizeof(float), s>>>(a);
     diff_stats_kernel<<<pairs, 256, size_t(2) * a.L * kStatStrip * sizeof(double), s>>>(a);
     B200_DIFF_DISPATCH(N, corr, a, pairs, s);
     ck(cudaGetLastError(), "the differentiable forward launches");
@@ -88,7 +87,8 @@ void launch_diff_backward(const DiffArgs &a, int N, cudaStream_t s)
     const unsigned pairs = pair_grid(a);
     if (!pairs) return;
     B200_DIFF_DISPATCH(N, adjoint, a, pairs, s);
-    diff_scatter_kernel<<<pairs, 256, 0, s>>>(a);
+    // at most 43 KB (L = 256)
+    diff_scatter_kernel<<<pairs, 256, size_t(kStripRows) * std::max(2 * a.L, a.L + kTaps - 1) * sizeof(float), s>>>(a);
     ck(cudaGetLastError(), "the differentiable backward launches");
 }
 

@@ -27,12 +27,47 @@ __device__ double chip_mean(const float *x, int L)
 // a frame index clamped to [0, n): the edge pixel repeats beyond the frame
 __device__ __forceinline__ int clamp_index(int i, int n) { return i < 0 ? 0 : (i >= n ? n - 1 : i); }
 
+// The interpolation is separable, and so is its transpose: the kernels below take strips of kStrip rows, the six
+// taps along the rows first, into shared memory (kStrip + 5 rows), then the six down the columns: 12
+// multiply-adds and 6 loads per pixel instead of 36 and 36 (the gather, bound by its loads and index clamps:
+// 91.6 to 57.0 us), and one atomic per frame pixel a chip touches instead of 36 per chip pixel (the scatter,
+// bound by its atomics: 234 to 122 us; both for 1,476 pairs of 80 x 80 chips). A warp takes a row, lanes along it.
+constexpr int kStrip = 16, kStripRows = kStrip + kTaps - 1;
+
+// sum_e w[e] F[row][x0 + kTap0 + j + e] (and the same of w2 if given) for the frame rows y .. y + kStripRows - 1,
+// j < L, into dst (kStripRows x L); rows and columns clamped to the frame
+template <bool TWO>
+__device__ __forceinline__ void strip_rows(const DiffArgs &a, const float *F, int y, int rows, int x0, const float (&w)[kTaps],
+                                           const float (&w2)[kTaps], float *dst, float *dst2)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, L = a.L;
+    const int c0 = x0 + kTap0;
+    const bool in = c0 >= 0 && c0 <= a.w - (L + kTaps - 1);
+    for (int i = warp; i < rows; i += nw) {
+        const float *r = F + int64_t(clamp_index(y + i, a.h)) * a.pitch;
+        for (int j = lane; j < L; j += 32) {
+            float f[kTaps];
+#pragma unroll
+            for (int e = 0; e < kTaps; ++e) f[e] = r[in ? c0 + j + e : clamp_index(c0 + j + e, a.w)];
+            float s = 0.0f, s2 = 0.0f;
+#pragma unroll
+            for (int e = 0; e < kTaps; ++e) {
+                s += w[e] * f[e];
+                if (TWO) s2 += w2[e] * f[e];
+            }
+            dst[i * L + j] = s;
+            if (TWO) dst2[i * L + j] = s2;
+        }
+    }
+}
+
 // the chips: one CTA per pair
 __global__ void __launch_bounds__(256) diff_gather_kernel(DiffArgs a)
 {
+    extern __shared__ float strip[];   // kStripRows x L
     const int64_t q = blockIdx.x;
     const DiffPair p = diff_pair(a, q);
-    const int L = a.L;
+    const int L = a.L, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     float *x = a.chips + q * L * L;
     if (!p.ok) {
         for (int i = threadIdx.x; i < L * L; i += blockDim.x) x[i] = 0.0f;
@@ -42,26 +77,24 @@ __global__ void __launch_bounds__(256) diff_gather_kernel(DiffArgs a)
     interp_weights(p.ay, wy, dw);
     interp_weights(p.ax, wx, dw);
     const float *F = a.frames + p.f * a.fstride;
-    for (int idx = threadIdx.x; idx < L * L; idx += blockDim.x) {
-        const int i = idx / L, j = idx % L;
-        int cx[kTaps];
+    for (int i0 = 0; i0 < L; i0 += kStrip) {
+        const int ni = min(kStrip, L - i0);
+        strip_rows<false>(a, F, p.y0 + kTap0 + i0, ni + kTaps - 1, p.x0, wx, wx, strip, nullptr);
+        __syncthreads();
+        for (int i = warp; i < ni; i += nw)
+            for (int j = lane; j < L; j += 32) {
+                float v = 0.0f;
 #pragma unroll
-        for (int e = 0; e < kTaps; ++e) cx[e] = clamp_index(p.x0 + kTap0 + j + e, a.w);
-        float v = 0.0f;
-#pragma unroll
-        for (int d = 0; d < kTaps; ++d) {
-            const float *r = F + int64_t(clamp_index(p.y0 + kTap0 + i + d, a.h)) * a.pitch;
-            float row = 0.0f;
-#pragma unroll
-            for (int e = 0; e < kTaps; ++e) row += wx[e] * r[cx[e]];
-            v += wy[d] * row;
-        }
-        x[idx] = v;
+                for (int d = 0; d < kTaps; ++d) v += wy[d] * strip[(i + d) * L + j];
+                x[(i0 + i) * L + j] = v;
+            }
+        __syncthreads();
     }
 }
 
 // the box statistics of each pair: (mu, 1 / s) for every (u, v), sums in FP64 over column strips
-constexpr int kStatStrip = 16;
+// (bound by the conversions of the pixels to FP64, so a row sum is taken once per kStatSlide boxes: 65.5 to 64.0 us)
+constexpr int kStatStrip = 16, kStatSlide = 4;
 __global__ void __launch_bounds__(256) diff_stats_kernel(DiffArgs a)
 {
     extern __shared__ double rs[];   // 2 x L x kStatStrip: row sums of x and x^2 over W columns
@@ -77,17 +110,26 @@ __global__ void __launch_bounds__(256) diff_stats_kernel(DiffArgs a)
     const double n = double(W) * W;
     double *r1 = rs, *r2 = rs + L * kStatStrip;
     for (int v0 = 0; v0 < M; v0 += kStatStrip) {
-        for (int idx = threadIdx.x; idx < L * kStatStrip; idx += blockDim.x) {
-            const int i = idx / kStatStrip, dv = idx % kStatStrip, v = v0 + dv;
+        // kStatSlide neighbours per thread: the first summed, the others by the pixels that enter and leave
+        for (int idx = threadIdx.x; idx < L * (kStatStrip / kStatSlide); idx += blockDim.x) {
+            const int i = idx / (kStatStrip / kStatSlide), dv = idx % (kStatStrip / kStatSlide) * kStatSlide, v = v0 + dv;
+            if (v >= M) continue;
             double s1 = 0.0, s2 = 0.0;
-            if (v < M)
-                for (int j = v; j < v + W; ++j) {
-                    const double e = x[i * L + j];
-                    s1 += e;
-                    s2 += e * e;
-                }
-            r1[idx] = s1;
-            r2[idx] = s2;
+            for (int j = v; j < v + W; ++j) {
+                const double e = x[i * L + j];
+                s1 += e;
+                s2 += e * e;
+            }
+            double *o1 = r1 + i * kStatStrip + dv, *o2 = r2 + i * kStatStrip + dv;
+            o1[0] = s1;
+            o2[0] = s2;
+            for (int t = 1; t < kStatSlide && v + t < M; ++t) {
+                const double in = x[i * L + v + t - 1 + W], out = x[i * L + v + t - 1];
+                s1 += in - out;
+                s2 += in * in - out * out;
+                o1[t] = s1;
+                o2[t] = s2;
+            }
         }
         __syncthreads();
         for (int idx = threadIdx.x; idx < M * kStatStrip; idx += blockDim.x) {
@@ -109,7 +151,7 @@ __global__ void __launch_bounds__(256) diff_stats_kernel(DiffArgs a)
 // the normalized surfaces and the peak outputs: one CTA per pair, the FFT passes of corr_kernel
 // on the float chip (minus its mean, which the zero-mean reference window does not see)
 template <int N, int NT>
-__global__ void __launch_bounds__(NT) diff_corr_kernel(DiffArgs a)
+__global__ void __launch_bounds__(NT, corr_blocks(N)) diff_corr_kernel(DiffArgs a)
 {
     using G = Geo<N>;
     extern __shared__ float4 smem_raw[];
@@ -151,7 +193,7 @@ __global__ void __launch_bounds__(NT) diff_corr_kernel(DiffArgs a)
 
 // the chip cotangents from the surface cotangents: one CTA per pair
 template <int N, int NT>
-__global__ void __launch_bounds__(NT) adjoint_kernel(DiffArgs a)
+__global__ void __launch_bounds__(NT, corr_blocks(N)) adjoint_kernel(DiffArgs a)
 {
     using G = Geo<N>;
     extern __shared__ float4 smem_raw[];
@@ -195,33 +237,74 @@ __global__ void __launch_bounds__(NT) adjoint_kernel(DiffArgs a)
     __syncthreads();
 
     // minus sum over the boxes holding p of B (x[p] - mu), B = G rho / s^2, as two box filters of
-    // B and B mu over the M x M grid (x and mu taken about the chip mean)
+    // B and B mu over the M x M grid (x and mu taken about the chip mean). Along the rows a warp scans a grid
+    // row in FP64 and takes differences; down the columns a thread sums the first position of its segment of
+    // kAdjointRows rows and slides. The chip's columns go in tiles whose two M x tile sums fit the FFT's tile
+    // of shared memory. (One thread per grid row and per column, in two passes, left the block waiting for
+    // its serial loops: 234 to 134 us, with the threads of corr_threads for 1,476 pairs of 80 x 80 chips.)
+    constexpr int kAdjointRows = 16;
     const float mean = float(chip_mean<NT>(x, L));
-    float *cb = Sr;   // M x L: the column-direction box sums
-    for (int pass = 0; pass < 2; ++pass) {
-        for (int u = threadIdx.x; u < M; u += NT) {
-            double s = 0.0;
-            for (int px = 0; px < L; ++px) {
-                for (int side = 0; side < 2; ++side) {
-                    const int v = side ? px - W : px;
-                    if (v < 0 || v >= M) continue;
-                    const int uv = u * M + v;
-                    const float is = st[2 * uv + 1];
-                    float b = gs[uv] * rho[uv] * is * is;
-                    if (pass == 1) b *= st[2 * uv] - mean;
-                    s += side ? -double(b) : double(b);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int NW = NT / 32;
+    double *P = reinterpret_cast<double *>(S) + warp * M;   // the warp's prefix sums
+    float2 *cb = S + NW * M;                                // M x tile: the sums along the rows of {B, B mu}
+    const int fit = (N * G::NHP - NW * M) / M, tile = min(L, fit >= 32 ? fit & ~31 : fit);
+    for (int p0 = 0; p0 < L; p0 += tile) {
+        const int np = min(tile, L - p0);
+        for (int u = warp; u < M; u += NW)
+            for (int pass = 0; pass < 2; ++pass) {
+                double carry = 0.0;
+                for (int v0 = 0; v0 < M; v0 += 32) {
+                    const int v = v0 + lane, uv = u * M + v;
+                    double b = 0.0;
+                    if (v < M) {
+                        const float is = st[2 * uv + 1];
+                        float t = gs[uv] * rho[uv] * is * is;
+                        if (pass == 1) t *= st[2 * uv] - mean;
+                        b = t;
+                    }
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const double t = __shfl_up_sync(0xffffffffu, b, o);
+                        if (lane >= o) b += t;
+                    }
+                    if (v < M) P[v] = carry + b;
+                    carry += __shfl_sync(0xffffffffu, b, 31);
                 }
-                cb[u * L + px] = float(s);
+                __syncwarp();
+                for (int c = lane; c < np; c += 32) {
+                    const int px = p0 + c, lo = px - W;
+                    const float t = float(P[min(px, M - 1)] - (lo >= 0 ? P[lo] : 0.0));
+                    if (pass == 0)
+                        cb[u * np + c].x = t;
+                    else
+                        cb[u * np + c].y = t;
+                }
+                __syncwarp();
             }
-        }
         __syncthreads();
-        for (int px = threadIdx.x; px < L; px += NT) {
-            double s = 0.0;
-            for (int py = 0; py < L; ++py) {
-                if (py < M) s += cb[py * L + px];
-                if (py - W >= 0 && py - W < M) s -= cb[(py - W) * L + px];
-                const int i = py * L + px;
-                gx[i] = pass == 0 ? float(gx[i] - (x[i] - mean) * s) : float(gx[i] + s);
+        const int npw = (np + 31) & ~31, segs = (L + kAdjointRows - 1) / kAdjointRows;
+        for (int idx = threadIdx.x; idx < segs * npw; idx += NT) {
+            const int c = idx % npw, y0 = idx / npw * kAdjointRows, y1 = min(L, y0 + kAdjointRows);
+            if (c >= np) continue;
+            double s0 = 0.0, s1 = 0.0;
+            for (int u = max(0, y0 - W); u < min(y0, M); ++u) {   // the grid rows over row y0 - 1
+                const float2 t = cb[u * np + c];
+                s0 += t.x;
+                s1 += t.y;
+            }
+            for (int py = y0; py < y1; ++py) {
+                if (py < M) {
+                    const float2 t = cb[py * np + c];
+                    s0 += t.x;
+                    s1 += t.y;
+                }
+                if (py - W >= 0 && py - W < M) {
+                    const float2 t = cb[(py - W) * np + c];
+                    s0 -= t.x;
+                    s1 -= t.y;
+                }
+                const int i = py * L + p0 + c;
+                gx[i] = float(float(gx[i] - (x[i] - mean) * s0) + s1);
             }
         }
         __syncthreads();
@@ -232,6 +315,7 @@ __global__ void __launch_bounds__(NT) adjoint_kernel(DiffArgs a)
 // per pair, frame cotangents accumulated atomically (windows overlap)
 __global__ void __launch_bounds__(256) diff_scatter_kernel(DiffArgs a)
 {
+    extern __shared__ float strip[];   // kStripRows x max(2 L, L + 5)
     __shared__ float red[2][8];
     const int64_t q = blockIdx.x;
     const DiffPair p = diff_pair(a, q);
@@ -247,31 +331,57 @@ __global__ void __launch_bounds__(256) diff_scatter_kernel(DiffArgs a)
     const float *F = a.frames + base;
     float *GF = a.g_frames ? a.g_frames + base : nullptr;
     const float *gx = a.g_chips + q * L * L;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     float ty = 0.0f, tx = 0.0f;
-    for (int idx = threadIdx.x; idx < L * L; idx += blockDim.x) {
-        const int i = idx / L, j = idx % L;
-        const float g = gx[idx];
-        if (g == 0.0f) continue;
-        int cx[kTaps];
+    if (a.g_shift)
+        for (int i0 = 0; i0 < L; i0 += kStrip) {
+            const int ni = min(kStrip, L - i0);
+            float *strip2 = strip + kStripRows * L;
+            strip_rows<true>(a, F, p.y0 + kTap0 + i0, ni + kTaps - 1, p.x0, wx, dx, strip, strip2);
+            __syncthreads();
+            for (int i = warp; i < ni; i += nw)
+                for (int j = lane; j < L; j += 32) {
+                    const float g = gx[(i0 + i) * L + j];
+                    if (g == 0.0f) continue;
+                    float sy = 0.0f, sx = 0.0f;
 #pragma unroll
-        for (int e = 0; e < kTaps; ++e) cx[e] = clamp_index(p.x0 + kTap0 + j + e, a.w);
-        float sy = 0.0f, sx = 0.0f;
-#pragma unroll
-        for (int d = 0; d < kTaps; ++d) {
-            const int64_t r = int64_t(clamp_index(p.y0 + kTap0 + i + d, a.h)) * a.pitch;
-            float row = 0.0f, drow = 0.0f;
-#pragma unroll
-            for (int e = 0; e < kTaps; ++e) {
-                const float fv = F[r + cx[e]];
-                row += wx[e] * fv;
-                drow += dx[e] * fv;
-                if (GF) atomicAdd(GF + r + cx[e], g * wy[d] * wx[e]);
-            }
-            sy += dy[d] * row;
-            sx += wy[d] * drow;
+                    for (int d = 0; d < kTaps; ++d) {
+                        sy += dy[d] * strip[(i + d) * L + j];
+                        sx += wy[d] * strip2[(i + d) * L + j];
+                    }
+                    ty += g * sy;
+                    tx += g * sx;
+                }
+            __syncthreads();
         }
-        ty += g * sy;
-        tx += g * sx;
+    if (GF) {
+        const int T = L + kTaps - 1;   // the chip's frame pixels: T x T from (y0 + kTap0, x0 + kTap0)
+        for (int r0 = 0; r0 < T; r0 += kStrip) {
+            const int nr = min(kStrip, T - r0);
+            // strip row t: the chip row r0 - 5 + t spread along the frame's columns
+            for (int t = warp; t < nr + kTaps - 1; t += nw) {
+                const int i = r0 - (kTaps - 1) + t;
+                for (int c = lane; c < T; c += 32) {
+                    float s = 0.0f;
+                    if (i >= 0 && i < L)
+#pragma unroll
+                        for (int e = 0; e < kTaps; ++e)
+                            if (c - e >= 0 && c - e < L) s += wx[e] * gx[i * L + c - e];
+                    strip[t * T + c] = s;
+                }
+            }
+            __syncthreads();
+            for (int t = warp; t < nr; t += nw) {
+                float *row = GF + int64_t(clamp_index(p.y0 + kTap0 + r0 + t, a.h)) * a.pitch;
+                for (int c = lane; c < T; c += 32) {
+                    float s = 0.0f;
+#pragma unroll
+                    for (int d = 0; d < kTaps; ++d) s += wy[d] * strip[(t + kTaps - 1 - d) * T + c];
+                    if (s != 0.0f) atomicAdd(row + clamp_index(p.x0 + kTap0 + c, a.w), s);
+                }
+            }
+            __syncthreads();
+        }
     }
     if (!a.g_shift) return;
     for (int o = 16; o > 0; o >>= 1) {
