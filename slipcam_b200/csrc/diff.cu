@@ -1,7 +1,6 @@
 // diff.cu -- the launches of the differentiable correlation (diff.cuh): one CTA per pair for
 // every stage; the FFT stages are instantiated for the FFT sizes of the correlation kernels.
 
-#include <algorithm>
 #include <stdexcept>
 #include <string>
 
@@ -76,7 +75,7 @@ void launch_diff_forward(const DiffArgs &a, int N, cudaStream_t s)
     const unsigned pairs = pair_grid(a);
     if (!pairs) return;
     B200_DIFF_DISPATCH(N, prepare);
-    diff_gather_kernel<<<pairs, 256, size_t(kStripRows) * a.L * sizeof(float), s>>>(a);
+    diff_gather_kernel<<<pairs, 256, 0, s>>>(a);
     diff_stats_kernel<<<pairs, 256, size_t(2) * a.L * kStatStrip * sizeof(double), s>>>(a);
     B200_DIFF_DISPATCH(N, corr, a, pairs, s);
     ck(cudaGetLastError(), "the differentiable forward launches");
@@ -87,8 +86,7 @@ void launch_diff_backward(const DiffArgs &a, int N, cudaStream_t s)
     const unsigned pairs = pair_grid(a);
     if (!pairs) return;
     B200_DIFF_DISPATCH(N, adjoint, a, pairs, s);
-    // at most 43 KB (L = 256)
-    diff_scatter_kernel<<<pairs, 256, size_t(kStripRows) * std::max(2 * a.L, a.L + kTaps - 1) * sizeof(float), s>>>(a);
+    diff_scatter_kernel<<<pairs, 256, 0, s>>>(a);
     ck(cudaGetLastError(), "the differentiable backward launches");
 }
 

@@ -27,36 +27,32 @@ __device__ double chip_mean(const float *x, int L)
 // a frame index clamped to [0, n): the edge pixel repeats beyond the frame
 __device__ __forceinline__ int clamp_index(int i, int n) { return i < 0 ? 0 : (i >= n ? n - 1 : i); }
 
-// The interpolation is separable, and so is its transpose: the kernels below take strips of kStrip rows, the six
-// taps along the rows first, into shared memory (kStrip + 5 rows), then the six down the columns: 12
-// multiply-adds and 6 loads per pixel instead of 36 and 36 (the gather, bound by its loads and index clamps:
-// 91.6 to 57.0 us), and one atomic per frame pixel a chip touches instead of 36 per chip pixel (the scatter,
-// bound by its atomics: 234 to 122 us; both for 1,476 pairs of 80 x 80 chips). A warp takes a row, lanes along it.
-constexpr int kStrip = 16, kStripRows = kStrip + kTaps - 1;
-
-// sum_e w[e] F[row][x0 + kTap0 + j + e] (and the same of w2 if given) for the frame rows y .. y + kStripRows - 1,
-// j < L, into dst (kStripRows x L); rows and columns clamped to the frame
-template <bool TWO>
-__device__ __forceinline__ void strip_rows(const DiffArgs &a, const float *F, int y, int rows, int x0, const float (&w)[kTaps],
-                                           const float (&w2)[kTaps], float *dst, float *dst2)
+// The interpolation is separable, and so is its transpose: in the kernels below a thread takes a column of a
+// chip and a segment of its rows, applies the six taps along each row as it comes and keeps the last six rows'
+// results in registers for the taps down the column: 12 multiply-adds and 6 loads per pixel instead of 36 and
+// 36 (the gather, bound by its instructions: 91.6 to 29.0 us), and one atomic per frame pixel that a segment touches
+// instead of 36 per chip pixel (the scatter: 234 to 67.9 us; both for 1,476 pairs of 80 x 80 chips). The segments fill
+// the block: blockDim / columns of them.
+__device__ __forceinline__ int column_rows(int cols, int rows)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, L = a.L;
-    const int c0 = x0 + kTap0;
-    const bool in = c0 >= 0 && c0 <= a.w - (L + kTaps - 1);
-    for (int i = warp; i < rows; i += nw) {
-        const float *r = F + int64_t(clamp_index(y + i, a.h)) * a.pitch;
-        for (int j = lane; j < L; j += 32) {
-            float f[kTaps];
+    const int segs = max(1, int(blockDim.x) / cols);
+    return (rows + segs - 1) / segs;
+}
+
+// for each row i of [i0, i1): out(i, ring), ring(d) the result of row(i + d), d < kTaps, for the rows
+// row(i0) .. row(i1 + kTaps - 2) in turn
+template <class T, class Row, class Out>
+__device__ __forceinline__ void slide_rows(int i0, int i1, Row &&row, Out &&out)
+{
+    T r[kTaps];
 #pragma unroll
-            for (int e = 0; e < kTaps; ++e) f[e] = r[in ? c0 + j + e : clamp_index(c0 + j + e, a.w)];
-            float s = 0.0f, s2 = 0.0f;
+    for (int d = 0; d < kTaps - 1; ++d) r[d] = row(i0 + d);
+    for (int i = i0; i < i1; i += kTaps) {
 #pragma unroll
-            for (int e = 0; e < kTaps; ++e) {
-                s += w[e] * f[e];
-                if (TWO) s2 += w2[e] * f[e];
-            }
-            dst[i * L + j] = s;
-            if (TWO) dst2[i * L + j] = s2;
+        for (int t = 0; t < kTaps; ++t) {
+            if (i + t >= i1) break;
+            r[(t + kTaps - 1) % kTaps] = row(i + t + kTaps - 1);
+            out(i + t, [&](int d) { return r[(t + d) % kTaps]; });
         }
     }
 }
@@ -64,10 +60,9 @@ __device__ __forceinline__ void strip_rows(const DiffArgs &a, const float *F, in
 // the chips: one CTA per pair
 __global__ void __launch_bounds__(256) diff_gather_kernel(DiffArgs a)
 {
-    extern __shared__ float strip[];   // kStripRows x L
     const int64_t q = blockIdx.x;
     const DiffPair p = diff_pair(a, q);
-    const int L = a.L, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int L = a.L;
     float *x = a.chips + q * L * L;
     if (!p.ok) {
         for (int i = threadIdx.x; i < L * L; i += blockDim.x) x[i] = 0.0f;
@@ -77,27 +72,39 @@ __global__ void __launch_bounds__(256) diff_gather_kernel(DiffArgs a)
     interp_weights(p.ay, wy, dw);
     interp_weights(p.ax, wx, dw);
     const float *F = a.frames + p.f * a.fstride;
-    for (int i0 = 0; i0 < L; i0 += kStrip) {
-        const int ni = min(kStrip, L - i0);
-        strip_rows<false>(a, F, p.y0 + kTap0 + i0, ni + kTaps - 1, p.x0, wx, wx, strip, nullptr);
-        __syncthreads();
-        for (int i = warp; i < ni; i += nw)
-            for (int j = lane; j < L; j += 32) {
+    const int rows = column_rows(L, L), segs = (L + rows - 1) / rows;
+    for (int idx = threadIdx.x; idx < segs * L; idx += blockDim.x) {
+        const int j = idx % L, i0 = idx / L * rows;
+        int cx[kTaps];
+#pragma unroll
+        for (int e = 0; e < kTaps; ++e) cx[e] = clamp_index(p.x0 + kTap0 + j + e, a.w);
+        slide_rows<float>(
+            i0, min(L, i0 + rows),
+            [&](int i) {
+                const float *r = F + int64_t(clamp_index(p.y0 + kTap0 + i, a.h)) * a.pitch;
+                float s = 0.0f;
+#pragma unroll
+                for (int e = 0; e < kTaps; ++e) s += wx[e] * r[cx[e]];
+                return s;
+            },
+            [&](int i, auto ring) {
                 float v = 0.0f;
 #pragma unroll
-                for (int d = 0; d < kTaps; ++d) v += wy[d] * strip[(i + d) * L + j];
-                x[(i0 + i) * L + j] = v;
-            }
-        __syncthreads();
+                for (int d = 0; d < kTaps; ++d) v += wy[d] * ring(d);
+                x[i * L + j] = v;
+            });
     }
 }
 
-// the box statistics of each pair: (mu, 1 / s) for every (u, v), sums in FP64 over column strips
-// (bound by the conversions of the pixels to FP64, so a row sum is taken once per kStatSlide boxes: 65.5 to 64.0 us)
-constexpr int kStatStrip = 16, kStatSlide = 4;
+// the box statistics of each pair: (mu, 1 / s) for every (u, v), sums in FP64 over strips of up to kStatStrip
+// grid rows: a thread takes a column of the chip and a segment of the strip, sums its first W pixels and slides
+// down; then kStatSlide neighbours along a grid row per thread, the first summed, the others by the column sums that
+// enter and leave (an odd number: the lanes' 8-byte reads are then conflict-free). Summing along the rows
+// first, W loads and conversions per box and row: 65.5 us, this way 30.7.
+constexpr int kStatStrip = 16, kStatSlide = 3;
 __global__ void __launch_bounds__(256) diff_stats_kernel(DiffArgs a)
 {
-    extern __shared__ double rs[];   // 2 x L x kStatStrip: row sums of x and x^2 over W columns
+    extern __shared__ double rs[];   // 2 x kStatStrip x L: column sums of x and x^2 over W rows
     const int64_t q = blockIdx.x;
     const DiffPair p = diff_pair(a, q);
     const int L = a.L, M = a.M, W = a.W;
@@ -108,41 +115,50 @@ __global__ void __launch_bounds__(256) diff_stats_kernel(DiffArgs a)
     }
     const float *x = a.chips + q * L * L;
     const double n = double(W) * W;
+    const int strips = (M + kStatStrip - 1) / kStatStrip, su = (M + strips - 1) / strips;
     double *r1 = rs, *r2 = rs + L * kStatStrip;
-    for (int v0 = 0; v0 < M; v0 += kStatStrip) {
-        // kStatSlide neighbours per thread: the first summed, the others by the pixels that enter and leave
-        for (int idx = threadIdx.x; idx < L * (kStatStrip / kStatSlide); idx += blockDim.x) {
-            const int i = idx / (kStatStrip / kStatSlide), dv = idx % (kStatStrip / kStatSlide) * kStatSlide, v = v0 + dv;
-            if (v >= M) continue;
+    for (int u0 = 0; u0 < M; u0 += su) {
+        const int nu = min(su, M - u0), rows = column_rows(L, nu), segs = (nu + rows - 1) / rows;
+        for (int idx = threadIdx.x; idx < segs * L; idx += blockDim.x) {
+            const int j = idx % L, t0 = idx / L * rows, t1 = min(nu, t0 + rows);
+            const float *c = x + (u0 + t0) * L + j;
             double s1 = 0.0, s2 = 0.0;
-            for (int j = v; j < v + W; ++j) {
-                const double e = x[i * L + j];
+#pragma unroll 8
+            for (int i = 0; i < W; ++i) {
+                const double e = c[i * L];
                 s1 += e;
                 s2 += e * e;
             }
-            double *o1 = r1 + i * kStatStrip + dv, *o2 = r2 + i * kStatStrip + dv;
-            o1[0] = s1;
-            o2[0] = s2;
-            for (int t = 1; t < kStatSlide && v + t < M; ++t) {
-                const double in = x[i * L + v + t - 1 + W], out = x[i * L + v + t - 1];
+            r1[t0 * L + j] = s1;
+            r2[t0 * L + j] = s2;
+            for (int t = t0 + 1; t < t1; ++t, c += L) {
+                const double in = c[W * L], out = c[0];
                 s1 += in - out;
                 s2 += in * in - out * out;
-                o1[t] = s1;
-                o2[t] = s2;
+                r1[t * L + j] = s1;
+                r2[t * L + j] = s2;
             }
         }
         __syncthreads();
-        for (int idx = threadIdx.x; idx < M * kStatStrip; idx += blockDim.x) {
-            const int u = idx / kStatStrip, dv = idx % kStatStrip, v = v0 + dv;
-            if (v >= M) continue;
+        const int ng = (M + kStatSlide - 1) / kStatSlide;
+        for (int idx = threadIdx.x; idx < nu * ng; idx += blockDim.x) {
+            const int t = idx / ng, v0 = idx % ng * kStatSlide;
+            const double *c1 = r1 + t * L + v0, *c2 = r2 + t * L + v0;
             double s1 = 0.0, s2 = 0.0;
-            for (int i = u; i < u + W; ++i) {
-                s1 += r1[i * kStatStrip + dv];
-                s2 += r2[i * kStatStrip + dv];
+            for (int j = 0; j < W; ++j) {
+                s1 += c1[j];
+                s2 += c2[j];
             }
-            const double var_n = s2 - s1 * s1 / n;   // n var
-            st[2 * (u * M + v)] = float(s1 / n);
-            st[2 * (u * M + v) + 1] = var_n > 0 ? float(1.0 / sqrt(var_n)) : 0.0f;
+            for (int k = 0; k < kStatSlide && v0 + k < M; ++k) {
+                if (k > 0) {
+                    s1 += c1[k - 1 + W] - c1[k - 1];
+                    s2 += c2[k - 1 + W] - c2[k - 1];
+                }
+                const double var_n = s2 - s1 * s1 / n;   // n var
+                const int uv = (u0 + t) * M + v0 + k;
+                st[2 * uv] = float(s1 / n);
+                st[2 * uv + 1] = var_n > 0 ? float(1.0 / sqrt(var_n)) : 0.0f;
+            }
         }
         __syncthreads();
     }
@@ -315,7 +331,6 @@ __global__ void __launch_bounds__(NT, corr_blocks(N)) adjoint_kernel(DiffArgs a)
 // per pair, frame cotangents accumulated atomically (windows overlap)
 __global__ void __launch_bounds__(256) diff_scatter_kernel(DiffArgs a)
 {
-    extern __shared__ float strip[];   // kStripRows x max(2 L, L + 5)
     __shared__ float red[2][8];
     const int64_t q = blockIdx.x;
     const DiffPair p = diff_pair(a, q);
@@ -331,56 +346,66 @@ __global__ void __launch_bounds__(256) diff_scatter_kernel(DiffArgs a)
     const float *F = a.frames + base;
     float *GF = a.g_frames ? a.g_frames + base : nullptr;
     const float *gx = a.g_chips + q * L * L;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     float ty = 0.0f, tx = 0.0f;
-    if (a.g_shift)
-        for (int i0 = 0; i0 < L; i0 += kStrip) {
-            const int ni = min(kStrip, L - i0);
-            float *strip2 = strip + kStripRows * L;
-            strip_rows<true>(a, F, p.y0 + kTap0 + i0, ni + kTaps - 1, p.x0, wx, dx, strip, strip2);
-            __syncthreads();
-            for (int i = warp; i < ni; i += nw)
-                for (int j = lane; j < L; j += 32) {
-                    const float g = gx[(i0 + i) * L + j];
-                    if (g == 0.0f) continue;
+    if (a.g_shift) {
+        const int rows = column_rows(L, L), segs = (L + rows - 1) / rows;
+        for (int idx = threadIdx.x; idx < segs * L; idx += blockDim.x) {
+            const int j = idx % L, i0 = idx / L * rows;
+            int cx[kTaps];
+#pragma unroll
+            for (int e = 0; e < kTaps; ++e) cx[e] = clamp_index(p.x0 + kTap0 + j + e, a.w);
+            slide_rows<float2>(
+                i0, min(L, i0 + rows),
+                [&](int i) {   // {F interpolated along the row, its derivative}
+                    const float *r = F + int64_t(clamp_index(p.y0 + kTap0 + i, a.h)) * a.pitch;
+                    float2 s = make_float2(0.0f, 0.0f);
+#pragma unroll
+                    for (int e = 0; e < kTaps; ++e) {
+                        const float f = r[cx[e]];
+                        s.x += wx[e] * f;
+                        s.y += dx[e] * f;
+                    }
+                    return s;
+                },
+                [&](int i, auto ring) {
+                    const float g = gx[i * L + j];
+                    if (g == 0.0f) return;
                     float sy = 0.0f, sx = 0.0f;
 #pragma unroll
                     for (int d = 0; d < kTaps; ++d) {
-                        sy += dy[d] * strip[(i + d) * L + j];
-                        sx += wy[d] * strip2[(i + d) * L + j];
+                        const float2 r = ring(d);
+                        sy += dy[d] * r.x;
+                        sx += wy[d] * r.y;
                     }
                     ty += g * sy;
                     tx += g * sx;
-                }
-            __syncthreads();
+                });
         }
+    }
     if (GF) {
         const int T = L + kTaps - 1;   // the chip's frame pixels: T x T from (y0 + kTap0, x0 + kTap0)
-        for (int r0 = 0; r0 < T; r0 += kStrip) {
-            const int nr = min(kStrip, T - r0);
-            // strip row t: the chip row r0 - 5 + t spread along the frame's columns
-            for (int t = warp; t < nr + kTaps - 1; t += nw) {
-                const int i = r0 - (kTaps - 1) + t;
-                for (int c = lane; c < T; c += 32) {
+        const int rows = column_rows(T, T), segs = (T + rows - 1) / rows;
+        for (int idx = threadIdx.x; idx < segs * T; idx += blockDim.x) {
+            const int c = idx % T, r0 = idx / T * rows;
+            const int col = clamp_index(p.x0 + kTap0 + c, a.w);
+            slide_rows<float>(
+                r0, min(T, r0 + rows),
+                [&](int t) {   // chip row t - 5 spread along the frame's columns
+                    const int i = t - (kTaps - 1);
                     float s = 0.0f;
                     if (i >= 0 && i < L)
 #pragma unroll
                         for (int e = 0; e < kTaps; ++e)
-                            if (c - e >= 0 && c - e < L) s += wx[e] * gx[i * L + c - e];
-                    strip[t * T + c] = s;
-                }
-            }
-            __syncthreads();
-            for (int t = warp; t < nr; t += nw) {
-                float *row = GF + int64_t(clamp_index(p.y0 + kTap0 + r0 + t, a.h)) * a.pitch;
-                for (int c = lane; c < T; c += 32) {
+                            if (unsigned(c - e) < unsigned(L)) s += wx[e] * gx[i * L + c - e];
+                    return s;
+                },
+                [&](int r, auto ring) {
                     float s = 0.0f;
 #pragma unroll
-                    for (int d = 0; d < kTaps; ++d) s += wy[d] * strip[(t + kTaps - 1 - d) * T + c];
-                    if (s != 0.0f) atomicAdd(row + clamp_index(p.x0 + kTap0 + c, a.w), s);
-                }
-            }
-            __syncthreads();
+                    for (int d = 0; d < kTaps; ++d) s += wy[kTaps - 1 - d] * ring(d);
+                    if (s != 0.0f)
+                        atomicAdd(GF + int64_t(clamp_index(p.y0 + kTap0 + r, a.h)) * a.pitch + col, s);
+                });
         }
     }
     if (!a.g_shift) return;
