@@ -28,6 +28,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/slipcam_b200.h"
+#include "dev_pool.h"
 
 namespace {
 
@@ -364,7 +365,7 @@ struct b200_stab {
     {
         for (void *p : {(void *)d_text, (void *)d_den, (void *)d_keep_idx, d_plans, (void *)d_work, (void *)d_blank,
                         (void *)d_vals, (void *)d_means})
-            if (p) cudaFree(p);
+            b200::dev_free(p);
     }
 };
 
@@ -407,6 +408,15 @@ PlanDev upload_plan(const PairwisePlan &p, char *&dst)
     return d;
 }
 
+template <class T>
+cudaError_t stab_alloc(T *&p, size_t bytes)
+{
+    void *q = nullptr;
+    const cudaError_t e = b200::dev_alloc(&q, bytes);
+    p = static_cast<T *>(q);
+    return e;
+}
+
 }   // namespace
 
 extern "C" {
@@ -437,23 +447,23 @@ int b200_stab_create(int height, int width, const uint8_t *text, int size, int d
             s->any_text = s->any_text || t[i];
         }
         const PairwisePlan pk = make_plan(int64_t(keep.size())), pa = make_plan(int64_t(px));
-        sck(cudaMalloc(&s->d_text, px), "cudaMalloc");
+        sck(stab_alloc(s->d_text, px), "cudaMalloc");
         sck(cudaMemcpy(s->d_text, t.data(), px, cudaMemcpyHostToDevice), "cudaMemcpy");
-        sck(cudaMalloc(&s->d_keep_idx, std::max<size_t>(keep.size(), 1) * 4), "cudaMalloc");
+        sck(stab_alloc(s->d_keep_idx, std::max<size_t>(keep.size(), 1) * 4), "cudaMalloc");
         if (!keep.empty())
             sck(cudaMemcpy(s->d_keep_idx, keep.data(), keep.size() * 4, cudaMemcpyHostToDevice), "cudaMemcpy");
-        sck(cudaMalloc(&s->d_plans, plan_bytes(pk) + plan_bytes(pa) + 256), "cudaMalloc");
+        sck(stab_alloc(s->d_plans, plan_bytes(pk) + plan_bytes(pa) + 256), "cudaMalloc");
         char *dst = static_cast<char *>(s->d_plans);
         s->plan_keep = upload_plan(pk, dst);
         s->plan_all = upload_plan(pa, dst);
         // frames per launch: about 64 MB of float32 work per buffer
         s->batch = int(std::clamp<int64_t>(int64_t(16) * 1024 * 1024 / int64_t(px), 1, 32));
         const size_t nodes = size_t(std::max(pk.leaf_start.size() + pk.left.size(), pa.leaf_start.size() + pa.left.size()));
-        sck(cudaMalloc(&s->d_den, px * 4), "cudaMalloc");
-        sck(cudaMalloc(&s->d_work, size_t(s->batch) * px * 4), "cudaMalloc");
-        sck(cudaMalloc(&s->d_blank, size_t(s->batch) * px * 4), "cudaMalloc");
-        sck(cudaMalloc(&s->d_vals, size_t(s->batch) * std::max<size_t>(nodes, 1) * 4), "cudaMalloc");
-        sck(cudaMalloc(&s->d_means, size_t(2) * s->batch * 4), "cudaMalloc");
+        sck(stab_alloc(s->d_den, px * 4), "cudaMalloc");
+        sck(stab_alloc(s->d_work, size_t(s->batch) * px * 4), "cudaMalloc");
+        sck(stab_alloc(s->d_blank, size_t(s->batch) * px * 4), "cudaMalloc");
+        sck(stab_alloc(s->d_vals, size_t(s->batch) * std::max<size_t>(nodes, 1) * 4), "cudaMalloc");
+        sck(stab_alloc(s->d_means, size_t(2) * s->batch * 4), "cudaMalloc");
         // den = uniform_filter(1 - text, size): the mask itself through the two passes
         if (box_rows_smem(size) > size_t(200) * 1024) throw StabFailure{B200_EINVAL, "framecor: the box is too large"};
         sck(cudaFuncSetAttribute(box_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(box_rows_smem(size))),
