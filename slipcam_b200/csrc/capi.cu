@@ -615,7 +615,7 @@ struct b200_handle {
             tc_refine_kernel<<<unsigned(int64_t(nwin) * cpw), 32 * wpc, rsm + size_t(wpc) * tsm, s>>>(a, d_refwin.p, d_sref.p,
                                                                                                      queue);
             const size_t psm = tc_patch_smem(W, M, stat);
-            tc_patch_kernel<<<unsigned(2 * num_sms()), 256, psm, s>>>(a, d_refwin.p, d_sref.p, queue);
+            tc_patch_kernel<<<unsigned(2 * num_sms()), kPatchThreads, psm, s>>>(a, d_refwin.p, d_sref.p, queue);
             CK(cudaGetLastError());
             launches += 2;
         }

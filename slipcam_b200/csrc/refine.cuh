@@ -59,32 +59,42 @@ __device__ __forceinline__ void stage_ref(unsigned char *dst, const uint8_t *ref
     }
 }
 
+// the frames' bytes [lo, hi): whole aligned words inside are read as such
+struct ByteRange {
+    uintptr_t lo, hi;
+};
+__device__ __forceinline__ ByteRange frame_bytes(const CorrArgs &a)
+{
+    const uint8_t *end = a.frames + int64_t(a.nf - 1) * a.fstride + int64_t(a.h - 1) * a.pitch + a.w;
+    return {reinterpret_cast<uintptr_t>(a.frames), reinterpret_cast<uintptr_t>(end)};
+}
+__device__ __forceinline__ uint32_t word_at(uintptr_t at, const ByteRange &in)
+{
+    if (at >= in.lo && at + 4 <= in.hi) return __ldg(reinterpret_cast<const uint32_t *>(at));
+    uint32_t v = 0;
+    for (int i = 0; i < 4; ++i)
+        if (at + i >= in.lo && at + i < in.hi) v |= uint32_t(__ldg(reinterpret_cast<const uint8_t *>(at + i))) << (8 * i);
+    return v;
+}
+
 // nr rows of nc bytes of the frame from src (row pitch `pitch`) into dst, rows of refine_tp(nc)
-// bytes; whole words when the frame rows start on 4-byte boundaries (every aligned word read holds
-// a byte of the region, so no read leaves the region's rows)
-__device__ __forceinline__ void stage_region(unsigned char *dst, const uint8_t *src, int64_t pitch, bool words, int nr,
+// bytes: two aligned words and a shift per word, whatever the rows' alignment (byte by byte, as unaligned
+// rows were staged before: with the sums sliding as on the 16-byte path 76.8 to 56.3 us at 477 x 853, window 48)
+__device__ __forceinline__ void stage_region(unsigned char *dst, const uint8_t *src, int64_t pitch, const ByteRange &in, int nr,
                                              int nc, int t, int nt)
 {
-    const int tp = refine_tp(nc), wpr = tp / 4;
-    if (words) {
-        uint32_t *d = reinterpret_cast<uint32_t *>(dst);
-        for (int e = t; e < nr * wpr; e += nt) {
-            const int r = e / wpr, w = e - r * wpr;
-            uint32_t v = 0;
-            if (4 * w < nc) {
-                const uintptr_t base = reinterpret_cast<uintptr_t>(src + int64_t(r) * pitch) + 4 * w;
-                const uint32_t *al = reinterpret_cast<const uint32_t *>(base & ~uintptr_t(3));
-                const int sh = int(base & 3);
-                const uint32_t lo = __ldg(al), hi = (sh != 0 && 4 * w + 4 - sh < nc) ? __ldg(al + 1) : 0u;
-                v = __funnelshift_r(lo, hi, 8 * sh);
-            }
-            d[e] = v;
+    const int wpr = refine_tp(nc) / 4;
+    uint32_t *d = reinterpret_cast<uint32_t *>(dst);
+    for (int e = t; e < nr * wpr; e += nt) {
+        const int r = e / wpr, w = e - r * wpr;
+        uint32_t v = 0;
+        if (4 * w < nc) {
+            const uintptr_t base = reinterpret_cast<uintptr_t>(src + int64_t(r) * pitch) + 4 * w, al = base & ~uintptr_t(3);
+            const int sh = int(base & 3);
+            const uint32_t lo = word_at(al, in), hi = (sh != 0 && 4 * w + 4 - sh < nc) ? word_at(al + 4, in) : 0u;
+            v = __funnelshift_r(lo, hi, 8 * sh);
         }
-    } else {
-        for (int e = t; e < nr * tp; e += nt) {
-            const int r = e / tp, c = e - r * tp;
-            dst[e] = c < nc ? __ldg(src + int64_t(r) * pitch + c) : 0;
-        }
+        d[e] = v;
     }
 }
 
@@ -141,7 +151,7 @@ __global__ void __launch_bounds__(256, 4) tc_refine_kernel(CorrArgs a, const uin
     if (!o.ok || !pi.valid || pi.u < 0 || pi.u >= M || pi.v < 0 || pi.v >= M) return;
     unsigned char *tile = smem + refine_ref_smem(W) + size_t(warp) * refine_tile_smem(W);
     const uint8_t *chip = a.frames + o.f * a.fstride + int64_t(o.sy) * a.pitch + o.sx;
-    const bool words = ((a.pitch | int(a.fstride & 3) | int(reinterpret_cast<uintptr_t>(a.frames) & 3)) & 3) == 0;
+    const ByteRange in = frame_bytes(a);
     const float scale = float(1.0 / (double(n) * double(a.norm[k])));
     const int2 *bt0 = a.bstat + size_t(o.f) * a.dinv_fstride + size_t(o.sy) * a.dpitch + o.sx;
     const int sr = sref[k];
@@ -172,40 +182,46 @@ __global__ void __launch_bounds__(256, 4) tc_refine_kernel(CorrArgs a, const uin
             }
             cp_wait_all();
         } else {
-            stage_region(tile, chip + int64_t(pu + u0) * a.pitch + pv + v0, a.pitch, words, nr, nc, lane, 32);
+            stage_region(tile, chip + int64_t(pu + u0) * a.pitch + pv + v0, a.pitch, in, nr, nc, lane, 32);
         }
         __syncwarp();
         uint32_t s[3][3] = {};
-        if (b16 && wpr <= 32) {
+        if (wpr <= 32) {
             // lane (w, rg) takes word column w of the reference rows ia .. ib - 1 and slides down them
             // with the three staged region rows of the 3 x 3 in registers: per row one reference word
             // and one new region row of three words
-            const int sw = sh >> 2, sb = sh & 3;   // the region's first word and byte in a staged row
+            const int sw = b16 ? sh >> 2 : 0, sb = b16 ? sh & 3 : 0;   // the region's first word and byte in a staged row
             const int nrg = 32 / wpr, rpl = (W + nrg - 1) / nrg;
             const int w = lane % wpr, rg = lane / wpr;
             const int ia = rg < nrg ? rg * rpl : W, ib = min(W, ia + rpl);
             if (ia < ib) {
                 const uint32_t *col = reinterpret_cast<const uint32_t *>(tile) + w + sw;
-                const int rw4 = rt >> 2;   // words per staged row
-                uint32_t a0 = col[ia * rw4], a1 = col[ia * rw4 + 1], a2 = col[ia * rw4 + 2];
-                uint32_t b0 = col[(ia + 1) * rw4], b1 = col[(ia + 1) * rw4 + 1], b2 = col[(ia + 1) * rw4 + 2];
-                for (int i = ia; i < ib; ++i) {
-                    const uint32_t *cr = col + (i + 2) * rw4;   // row i + 2 (inside the W + 2 staged rows)
-                    const uint32_t c0 = cr[0], c1 = cr[1], c2 = cr[2];
-                    const uint32_t rw = *reinterpret_cast<const uint32_t *>(sref_w + i * W + 4 * w);
+                const int rw4 = (b16 ? rt : tp) >> 2;   // words per staged row
+                // a row's bytes at the three shifts, once per row (177 to 127 us at 720p, window 64, when each was shifted for all nine sums)
+                auto shifts = [&](int r, uint32_t (&y)[3]) {
+                    const uint32_t *cr = col + r * rw4;
+                    const uint32_t w0 = cr[0], w1 = cr[1], w2 = cr[2];
+                    const uint32_t hi = __funnelshift_r(w1, w2, 8 * sb);
+                    y[0] = __funnelshift_r(w0, w1, 8 * sb);
+                    y[1] = __funnelshift_r(y[0], hi, 8);
+                    y[2] = __funnelshift_r(y[0], hi, 16);
+                };
+                uint32_t y[3][3];   // the rows in turn
+                shifts(ia, y[0]);
+                shifts(ia + 1, y[1]);
+                for (int ib3 = ia; ib3 < ib; ib3 += 3) {
 #pragma unroll
-                    for (int d = 0; d < 3; ++d) {
-                        if (d > v1 - v0) continue;
-                        s[0][d] = __dp4a(rw, bytes_at(a0, a1, a2, sb + d), s[0][d]);
-                        if (u1 - u0 >= 1) s[1][d] = __dp4a(rw, bytes_at(b0, b1, b2, sb + d), s[1][d]);
-                        if (u1 - u0 >= 2) s[2][d] = __dp4a(rw, bytes_at(c0, c1, c2, sb + d), s[2][d]);
+                    for (int t = 0; t < 3; ++t) {
+                        const int i = ib3 + t;
+                        if (i >= ib) break;
+                        shifts(i + 2, y[(t + 2) % 3]);   // row i + 2 (inside the W + 2 staged rows)
+                        const uint32_t rw = *reinterpret_cast<const uint32_t *>(sref_w + i * refine_rp(W) + 4 * w);
+                        // (at the surface's edge the sums of the shifts outside it are not read)
+#pragma unroll
+                        for (int du = 0; du < 3; ++du)
+#pragma unroll
+                            for (int d = 0; d < 3; ++d) s[du][d] = __dp4a(rw, y[(t + du) % 3][d], s[du][d]);
                     }
-                    a0 = b0;
-                    a1 = b1;
-                    a2 = b2;
-                    b0 = c0;
-                    b1 = c1;
-                    b2 = c2;
                 }
             }
         } else if (b16) {
@@ -289,15 +305,17 @@ __global__ void __launch_bounds__(256, 4) tc_refine_kernel(CorrArgs a, const uin
 
 // the SNR patch of each queued pair summed exactly: one CTA per pair, the reference window and the
 // patch's chip region in shared memory, a thread per patch position (dp4a over the reference rows'
-// words), then the pair's outputs
-__global__ void __launch_bounds__(256) tc_patch_kernel(CorrArgs a, const uint8_t *refwin, const int *sref,
+// words), then the pair's outputs. 448 threads: the 21 x 21 patch in one round: 43.9 to 39.3 us at 720p, window 64; 26.7
+// to 19.4 at 477 x 853, window 48
+constexpr int kPatchThreads = 448;
+__global__ void __launch_bounds__(kPatchThreads) tc_patch_kernel(CorrArgs a, const uint8_t *refwin, const int *sref,
                                                        const int *queue)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ double s_sum[8];
+    __shared__ double s_sum[kPatchThreads / 32];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int W = a.W, M = a.M, n = W * W, rp = refine_rp(W), wpr = rp / 4;
-    const bool words = ((a.pitch | int(a.fstride & 3) | int(reinterpret_cast<uintptr_t>(a.frames) & 3)) & 3) == 0;
+    const ByteRange in = frame_bytes(a);
     const int count = queue[0];
     unsigned char *sref_w = smem, *tile = smem + size_t(W) * rp;
     for (int t = blockIdx.x; t < count; t += gridDim.x) {
@@ -310,21 +328,27 @@ __global__ void __launch_bounds__(256) tc_patch_kernel(CorrArgs a, const uint8_t
         snr_patch(M, a.stat, pu, pv, i0, i1, j0, j1);
         const int pw = j1 - j0, np = (i1 - i0) * pw;
         const int nr = i1 - i0 + W - 1, nc = pw + W - 1, tp = refine_tp(nc);
-        stage_ref(sref_w, refwin + size_t(k) * W * W, W, tid, 256);
-        stage_region(tile, a.frames + o.f * a.fstride + int64_t(o.sy + i0) * a.pitch + o.sx + j0, a.pitch, words, nr, nc,
-                     tid, 256);
+        stage_ref(sref_w, refwin + size_t(k) * W * W, W, tid, kPatchThreads);
+        stage_region(tile, a.frames + o.f * a.fstride + int64_t(o.sy + i0) * a.pitch + o.sx + j0, a.pitch, in, nr, nc,
+                     tid, kPatchThreads);
         __syncthreads();
         const float scale = float(1.0 / (double(n) * double(a.norm[k])));
         const int2 *bt0 = a.bstat + size_t(o.f) * a.dinv_fstride + size_t(o.sy) * a.dpitch + o.sx;
         double sum = 0.0;
-        for (int q = tid; q < np; q += 256) {
+        for (int q = tid; q < np; q += kPatchThreads) {
             const int du = q / pw, dv = q - du * pw;
             const int sh = 8 * (dv & 3);
             uint32_t acc = 0;
             for (int i = 0; i < W; ++i) {
                 const uint32_t *rr = reinterpret_cast<const uint32_t *>(sref_w + i * rp);
                 const uint32_t *cr = reinterpret_cast<const uint32_t *>(tile + (du + i) * tp + (dv & ~3));
-                for (int w = 0; w < wpr; ++w) acc = __dp4a(rr[w], __funnelshift_r(cr[w], cr[w + 1], sh), acc);
+                uint32_t lo = cr[0];
+#pragma unroll 4
+                for (int w = 0; w < wpr; ++w) {
+                    const uint32_t hi = cr[w + 1];
+                    acc = __dp4a(rr[w], __funnelshift_r(lo, hi, sh), acc);
+                    lo = hi;
+                }
             }
             const float x = i8::rho(acc, __ldg(bt0 + int64_t(i0 + du) * a.dpitch + j0 + dv), n, sref[k], scale);
             sum += double(x) * double(x);
@@ -334,7 +358,7 @@ __global__ void __launch_bounds__(256) tc_patch_kernel(CorrArgs a, const uint8_t
         __syncthreads();
         if (tid == 0) {
             double tot = 0.0;
-            for (int w = 0; w < 8; ++w) tot += s_sum[w];
+            for (int w = 0; w < kPatchThreads / 32; ++w) tot += s_sum[w];
             peak_outputs(pi.fit + 4, 3, M, pu, pv, a.R, o.gy, o.gx, n, tot, np, p, a.offset, a.peak, a.snr, a.cov);
         }
         __syncthreads();   // the shared memory is the next pair's
