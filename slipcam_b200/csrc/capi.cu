@@ -855,11 +855,13 @@ DiffArgs diff_args(b200_handle *h, const float *frames, int n, int pitch, const 
 
 void b200::tc_dft_table(int N, uint16_t *out)
 {
+    // the N angles once (each a pair of series), not once per element: 1 ms of a handle's creation at N = 160
+    std::vector<double> cs(2 * size_t(N));
+    for (int k = 0; k < N; ++k) cs2pi(k, N, cs[2 * k], cs[2 * k + 1]);
     for (int r = 0; r < tc_rt(N); ++r)
         for (int c = 0; c < N; ++c) {
-            double cc = 0.0, sn = 0.0;
-            cs2pi(long(r < N / 2 ? r : r - N / 2) * c, N, cc, sn);
-            double v = r < N / 2 ? cc : r <= N ? -sn : 0.0;
+            const int k = int((long(r < N / 2 ? r : r - N / 2) * c) % N);
+            double v = r < N / 2 ? cs[2 * k] : r <= N ? -cs[2 * k + 1] : 0.0;
             if (r == N / 2) v = c % 2 ? -1.0 : 1.0;   // the Nyquist row, where S's row 0 would be
             out[tc_table_offset(N, r, c) / 2] = __half_as_ushort(__float2half_rn(float(v)));
         }
