@@ -56,11 +56,12 @@ def fft_flops(n):
 
 def tc_flops(n, m):
     """executed tensor-core FLOPs of one window in the DFT-GEMM form (FFT size n, m shifts per
-    axis): the five GEMM stages with their 128-row tiles and 16-column padding"""
+    axis): the five GEMM stages with their 128-row tiles and 16-column padding, half of the products of
+    the two complex stages by the symmetry of the DFT matrices"""
     kp = (n // 2 + 1 + 15) // 16 * 16
     no = (m + 15) // 16 * 16
-    t1 = (n + 127) // 128
-    return 4 * 128 * t1 * kp * n + 8 * 128 * n * n + 8 * 128 * no * n + 4 * 128 * no * kp
+    return 3 * 4 * 128 * n * n + 4 * 128 * no * kp
+
 
 
 class Clocks:
