@@ -13,17 +13,32 @@
 #include <algorithm>
 #include <cstdint>
 #include <mutex>
+#include <unordered_set>
 
 #include <cuda_runtime.h>
 
 namespace b200 {
 
 constexpr uint64_t kPoolKeep = uint64_t(1) << 30;
+// Larger buffers come from cudaMalloc: the pool could not keep two of them, and maps them more slowly (the 3.6 GB
+// of spectra of a dense 1080p grid: a handle made in 27 ms from the pool, in 7 ms from cudaMalloc).
+constexpr size_t kPoolBuffer = size_t(512) << 20;
 
 struct DevPool {
     cudaMemPool_t pool = nullptr;
     cudaStream_t stream = nullptr;   // orders the pool's allocations and releases; no work runs on it
 };
+
+// the buffers above kPoolBuffer, so that a release knows them
+struct DirectBuffers {
+    std::mutex mutex;
+    std::unordered_set<void *> held;
+};
+inline DirectBuffers &direct_buffers()
+{
+    static DirectBuffers *d = new DirectBuffers;   // outlives every handle
+    return *d;
+}
 
 // the current device's pool (pool == nullptr: it has none), and the device's index
 inline cudaError_t device_pool(DevPool &out, int &dev)
@@ -67,6 +82,19 @@ inline cudaError_t dev_alloc(void **p, size_t bytes)
     int dev = 0;
     if (cudaError_t e = device_pool(d, dev)) return e;
     if (!d.pool) return cudaMalloc(p, bytes);
+    if (bytes > kPoolBuffer) {
+        cudaError_t e = cudaMalloc(p, bytes);
+        if (e == cudaErrorMemoryAllocation) {   // what the pool holds unused first
+            cudaGetLastError();
+            cudaMemPoolTrimTo(d.pool, 0);
+            e = cudaMalloc(p, bytes);
+        }
+        if (e) return e;
+        DirectBuffers &b = direct_buffers();
+        std::lock_guard<std::mutex> lock(b.mutex);
+        b.held.insert(*p);
+        return cudaSuccess;
+    }
     cudaError_t e = cudaMallocFromPoolAsync(p, bytes, d.pool, d.stream);
     if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
@@ -92,7 +120,13 @@ inline void dev_free(void *p)
     DevPool d;
     int dev = 0;
     if (device_pool(d, dev) == cudaSuccess) {
-        if (!d.pool)
+        bool direct = !d.pool;
+        if (!direct) {
+            DirectBuffers &b = direct_buffers();
+            std::lock_guard<std::mutex> lock(b.mutex);
+            direct = b.held.erase(p) > 0;
+        }
+        if (direct)
             cudaFree(p);
         else if (cudaDeviceSynchronize() == cudaSuccess)
             cudaFreeAsync(p, d.stream);
