@@ -31,7 +31,7 @@ __device__ __forceinline__ int clamp_index(int i, int n) { return i < 0 ? 0 : (i
 // chip and a segment of its rows, applies the six taps along each row as it comes and keeps the last six rows'
 // results in registers for the taps down the column: 12 multiply-adds and 6 loads per pixel instead of 36 and
 // 36 (the gather, bound by its instructions: 91.6 to 29.0 us), and one atomic per frame pixel that a segment touches
-// instead of 36 per chip pixel (the scatter: 234 to 67.9 us; both for 1,476 pairs of 80 x 80 chips). The segments fill
+// instead of 36 per chip pixel (the scatter: 234 to 67.9 us; both for 1,025 pairs of 80 x 80 chips). The segments fill
 // the block: blockDim / columns of them.
 __device__ __forceinline__ int column_rows(int cols, int rows)
 {
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(NT, corr_blocks(N)) adjoint_kernel(DiffArgs a)
     // row in FP64 and takes differences; down the columns a thread sums the first position of its segment of
     // kAdjointRows rows and slides. The chip's columns go in tiles whose two M x tile sums fit the FFT's tile
     // of shared memory. (One thread per grid row and per column, in two passes, left the block waiting for
-    // its serial loops: 234 to 134 us, with the threads of corr_threads for 1,476 pairs of 80 x 80 chips.)
+    // its serial loops: 234 to 134 us, with the threads of corr_threads for 1,025 pairs of 80 x 80 chips.)
     constexpr int kAdjointRows = 16;
     const float mean = float(chip_mean<NT>(x, L));
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
