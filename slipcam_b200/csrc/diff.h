@@ -10,7 +10,7 @@
 //   stats   S1, S2 = sums of x, x^2 over the W x W box at (u, v); mu = S1 / n,
 //           s(u, v) = sqrt(S2 - S1^2 / n) in FP64 (the reference's sqrt((n S2 - S1^2) / n))
 //   surface rho(u, v) = c(u, v) / (norm s(u, v)), c(u, v) = sum_{i,j < W} r0[i][j] x[u + i][v + j]
-//           (0 where s = 0), c from the FP32 FFT passes against the resident reference spectra
+//           (0 where s is 0 within the rounding of S1 and S2), c from the FP32 FFT passes against the resident reference spectra
 //   peak    the reference's argmax, 3 x 3 fit, SNR and covariance (corr_fft.cuh)
 // Backward, from a cotangent G of the surface:
 //   dL/dx[p] = sum_{u,v} A(u, v) r0[p - (u, v)] - sum_{(u,v): p in box(u,v)} B(u, v) (x[p] - mu(u, v))
@@ -72,7 +72,7 @@ struct DiffArgs {
     int gross_mode;
     const float *shift;        // nullptr or n x nwin x 2: (ty, tx) of each pair
     float *chips;              // n x nwin x L x L
-    float *stats;              // n x nwin x M x M x 2: (mu, 1 / s) of each box (1 / s = 0 if s = 0)
+    float *stats;              // n x nwin x M x M x 2: (mu, 1 / s) of each box (1 / s = 0 if flat)
     float *surface;            // n x nwin x M x M
     int *peak_at;              // n x nwin: u M + v of the peak, or -1
     float *offset, *peak, *snr, *cov;
