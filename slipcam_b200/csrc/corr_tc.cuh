@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) corr_tc_kernel(const __grid_con
     __shared__ int s_abort;
     __shared__ PairSetup ring[4];      // the pairs in flight: gathered, drained, in the epilogue
     __shared__ uint32_t s_good[5];     // the events the relay has told of (wake)
-    __shared__ uint32_t s_taken;       // the pairs whose epilogue's turn the gather warps have passed
+    __shared__ uint32_t s_taken;       // the pairs whose entries the epilogue has read to the end
     __shared__ int s_key[kTcEpi], s_peak;   // the warps' largest values (as ints), the peak u M + v
     __shared__ long long s_sq[kTcEpi];
     __shared__ double s_wide;          // the part of the patch sum whose values do not fit the integers' range
@@ -968,11 +968,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) corr_tc_kernel(const __grid_con
                 for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
             }
             if (lane == 0) s_sq[ew] = sq;
+            // the last reads of the entry: the barrier is between them and the store below, which lets the setup warp
+            // overwrite it (without one the compiler may move these plain loads past the store)
+            const int64_t q = e.q;
+            const int gy = e.gy, gx = e.gx;
             asm volatile("bar.sync 1, %0;" ::"n"(32 * kTcEpi) : "memory");
             if (ew == 0 && lane == 0) {
-                const int64_t q = e.q;
-                const int gy = e.gy, gx = e.gx;
-                *const_cast<volatile uint32_t *>(&s_taken) = n + 1;   // nobody reads the entry any more
+                *const_cast<volatile uint32_t *>(&s_taken) = n + 1;
                 s_peak = INT_MAX;
                 if (!valid) {
                     tc_invalid(&a, q);
