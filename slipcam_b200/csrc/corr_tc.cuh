@@ -427,19 +427,32 @@ __device__ __forceinline__ void tc_gather(const CorrArgs &a, const PairSetup &c,
     }
 }
 
-// the entry of the CTA's pair n, as soon as it is written; false if a role gave up
+// The entry of the CTA's pair n, as soon as it is written; false if a role gave up. Called by whole warps, whose
+// lanes vote at each poll: all leave at the same one with the same answer, also when an abort and the entry
+// come about between the lanes' reads. (Bounded by the abort flag: a kernel that comes to a stop has a wait in the control
+// warp, and that one gives up.)
 __device__ __forceinline__ bool tc_entry(const PairSetup &e, uint32_t n, const volatile int *abort)
 {
-    bool ok = true;
-    while (*const_cast<const volatile uint32_t *>(&e.seq) != n + 1) {
-        if (*abort) {
-            ok = false;
-            break;
-        }
+    for (;;) {
+        const bool there = *const_cast<const volatile uint32_t *>(&e.seq) == n + 1;
+        const bool stop = !there && *abort;
+        if (__all_sync(0xffffffffu, there)) break;
+        if (__any_sync(0xffffffffu, stop)) return false;
         __nanosleep(64);
     }
     asm volatile("" ::: "memory");   // shared-memory reads stay in order
-    return __all_sync(__activemask(), ok);
+    return true;
+}
+
+// the same for a thread by itself
+__device__ __forceinline__ bool tc_entry_one(const PairSetup &e, uint32_t n, const volatile int *abort)
+{
+    while (*const_cast<const volatile uint32_t *>(&e.seq) != n + 1) {
+        if (*abort) return false;
+        __nanosleep(64);
+    }
+    asm volatile("" ::: "memory");
+    return true;
 }
 
 template <int N>
@@ -685,7 +698,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) corr_tc_kernel(const __grid_con
             uint32_t g = 0;   // chunks so far: slot g % 4, its use g / 4
             for (uint32_t n = 0;; ++n) {
                 const PairSetup &e = ring[n & 3];
-                if (!tc_entry(e, n, ab) || e.end) break;
+                if (!tc_entry_one(e, n, ab) || e.end) break;
                 const float4 *r = a.spec_tc + size_t(e.k) * (N / 2) * KP;
                 if (n && !tc_wait(&bar.stage[2], (n - 1) & 1u, ab)) break;   // S5 has read what the ring overwrites
                 bool ok = true;

@@ -22,3 +22,10 @@ def test_entry_is_read_before_it_is_given_back():
     end = text.index('\n    } else {\n', stores[0])   # of the epilogue's role
     assert not re.search(r'\be\.\w', text[barrier:end])
     assert re.search(r'\be\.q\b', text[:barrier])
+
+
+def test_a_warp_decides_as_one():
+    """No vote over the lanes that happen to be active: whole warps vote with the full mask, a lane by itself not at all."""
+    text = code()
+    assert '__activemask' not in text
+    assert text.count('tc_entry_one(e, n, ab)') == 1 and re.search(r'if \(lane == 0\) \{[^{}]*(\{[^{}]*)?tc_entry_one\(e, n, ab\)', text)
