@@ -469,8 +469,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) corr_tc_kernel(const __grid_con
     __shared__ uint32_t s_good[5];     // the events the relay has told of (wake)
     __shared__ uint32_t s_taken;       // the pairs whose entries the epilogue has read to the end
     __shared__ int s_key[kTcEpi], s_peak;   // the warps' largest values (as ints), the peak u M + v
-    __shared__ long long s_sq[kTcEpi];
-    __shared__ double s_wide;          // the part of the patch sum whose values do not fit the integers' range
+    __shared__ double s_sq[kTcEpi];
     __shared__ float s_fit[9];
     constexpr int kRowWarps = (KP + 31) / 32;   // drain warps with rows, of each part
     // the same on every lane, and known to be: the roles' branches are uniform
@@ -489,7 +488,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) corr_tc_kernel(const __grid_con
         s_taken = 0;
         for (int i = 0; i < 5; ++i) s_good[i] = 0;
         s_peak = INT_MAX;
-        s_wide = 0.0;
         tc::mbar_init(&bar.xfull, kTcGather);
         tc::mbar_init(&bar.xfree, 1);
         tc::mbar_init(&bar.stage[1], 1);
@@ -922,27 +920,21 @@ __global__ void __launch_bounds__(kTcThreads, 1) corr_tc_kernel(const __grid_con
             asm volatile("bar.sync 1, %0;" ::"n"(32 * kTcEpi) : "memory");
             const int at = valid ? s_peak : 0, pu = at / M, pv = at - pu * M;
             int i0 = 0, i1 = 0, j0 = 0, j1 = 0;
-            // the SNR patch's sum of squares and the 3 x 3 values, with the same arithmetic. The values are
-            // summed as integers, rounded to 2^-sh with sh as large as the patch's count allows (26 at 21 x
-            // 21: below FP32's own rounding of a value above 1/8), each product and the sum exact.
-            long long sq = 0;
-            int sh = 0;
+            // the SNR patch's sum of squares (of the FP32 values, in FP64) and the 3 x 3 values, with the same
+            // arithmetic
+            double sq = 0.0;
             auto release = [&] {   // this warp reads c's columns no more
                 tc::fence_before_sync();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&bar.cfree);
             };
-            if (valid) {
-                snr_patch(M, a.stat, pu, pv, i0, i1, j0, j1);
-                sh = (29 + __clz((i1 - i0) * (j1 - j0))) >> 1;   // count 4 2^(2 sh) < 2^63
-            }
+            if (valid) snr_patch(M, a.stat, pu, pv, i0, i1, j0, j1);
             // the warp's first group with a row of the patch, if it holds columns of it (warp-uniform)
             const bool cols = valid && 32 * quad < j1 && 32 * quad + 32 > j0;
             int u0 = 8 * part + (max(i0 - 7 - 8 * part, 0) + 15) / 16 * 16;
             if (!cols || u0 >= i1) {
                 release();
             } else {
-                const float up = __int_as_float((127 + sh) << 23);
                 const bool col = v >= j0 && v < j1;
                 const uint32_t fv = uint32_t(v - pv + 1);
 #pragma unroll 1
@@ -954,26 +946,17 @@ __global__ void __launch_bounds__(kTcThreads, 1) corr_tc_kernel(const __grid_con
                     if (u0 + 32 >= i1) release();
 #pragma unroll 1
                     for (int ub = u0; ub < u0 + 32; ub += 16) {
-                        bool wide = false;
+                        // two chains of FP64 (one: 2507 us for 16 720p frames against 2498; four: the same as two)
+                        double even = 0.0, odd = 0.0;
 #pragma unroll
                         for (int t = 0; t < 8; ++t) {
                             const uint32_t fu = uint32_t(ub + t - pu + 1);
                             float x = d0[t];
                             if (fu < 3u && fv < 3u) s_fit[fu * 3 + fv] = x;
                             if (!col || ub + t < i0 || ub + t >= i1) x = 0.0f;
-                            const int z = __float2int_rn(x * up);
-                            sq += (long long)z * z;
-                            wide |= !(fabsf(x) < 2.0f);
-                            d0[t] = x;
+                            (t & 1 ? odd : even) += double(x) * double(x);
                         }
-                        if (__any_sync(0xffffffffu, wide)) {   // values of 2 and more, or none: in FP64
-#pragma unroll
-                            for (int t = 0; t < 8; ++t) {
-                                const int z = __float2int_rn(d0[t] * up);
-                                sq -= (long long)z * z;
-                                if (d0[t] != 0.0f) atomicAdd(&s_wide, double(d0[t]) * double(d0[t]));
-                            }
-                        }
+                        sq += even + odd;
 #pragma unroll
                         for (int t = 0; t < 8; ++t) d0[t] = d1[t];
                     }
@@ -992,11 +975,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) corr_tc_kernel(const __grid_con
                 if (!valid) {
                     tc_invalid(&a, q);
                 } else {
-                    long long total = 0;
+                    double sum = 0.0;
 #pragma unroll 1
-                    for (int w = 0; w < kTcEpi; ++w) total += s_sq[w];
-                    const double sum = double(total) * __hiloint2double((1023 - 2 * sh) << 20, 0) + s_wide;
-                    s_wide = 0.0;
+                    for (int w = 0; w < kTcEpi; ++w) sum += s_sq[w];
                     const int count = (i1 - i0) * (j1 - j0);
                     if (a.peaks) {   // for the exact refinement of the peak, which writes the pair's outputs
                         PeakInfo &pi = a.peaks[q];
