@@ -7,7 +7,8 @@
 // of memory an allocation first returns all that is unused. The CUDA pool serves several threads and devices.
 //
 // The buffers are ready for, and freed after, every stream, as with cudaMalloc and cudaFree: an allocation
-// waits for its (empty) stream, a release first for the device. The contents of a buffer are undefined.
+// waits for its (empty) stream, a release first for the device (wait_for_device). The contents of a buffer are
+// undefined.
 #pragma once
 
 #include <algorithm>
@@ -24,9 +25,12 @@ constexpr uint64_t kPoolKeep = uint64_t(1) << 30;
 // of spectra of a dense 1080p grid: a handle made in 27 ms from the pool, in 7 ms from cudaMalloc).
 constexpr size_t kPoolBuffer = size_t(512) << 20;
 
+constexpr size_t kWaitBuffer = 256;
+
 struct DevPool {
     cudaMemPool_t pool = nullptr;
     cudaStream_t stream = nullptr;   // orders the pool's allocations and releases; no work runs on it
+    void *anchor = nullptr;          // keeps a block of small buffers mapped for wait_for_device
 };
 
 // the buffers above kPoolBuffer, so that a release knows them
@@ -63,6 +67,7 @@ inline cudaError_t device_pool(DevPool &out, int &dev)
             if (cudaMemPoolCreate(&p.pool, &props) == cudaSuccess &&
                 cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess &&
                 cudaStreamCreateWithFlags(&p.stream, cudaStreamNonBlocking) == cudaSuccess) {
+                if (cudaMalloc(&p.anchor, kWaitBuffer) != cudaSuccess) cudaGetLastError();
                 pools[dev] = p;
             } else {
                 cudaGetLastError();
@@ -73,6 +78,17 @@ inline cudaError_t device_pool(DevPool &out, int &dev)
     }
     out = pools[dev];
     return cudaSuccess;
+}
+
+// All work of the current device is done: cudaFree of a small buffer waits for it (5 us with the device idle, as long as
+// cudaDeviceSynchronize takes). Unlike that call it may be made while a stream is captured in the relaxed mode,
+// which a handle that goes must not end.
+inline bool wait_for_device()
+{
+    void *p = nullptr;
+    if (cudaMalloc(&p, kWaitBuffer) == cudaSuccess) return cudaFree(p) == cudaSuccess;
+    cudaGetLastError();
+    return cudaDeviceSynchronize() == cudaSuccess;
 }
 
 // bytes of device memory on the current device, for every stream
@@ -128,9 +144,9 @@ inline void dev_free(void *p)
         }
         if (direct)
             cudaFree(p);
-        else if (cudaDeviceSynchronize() == cudaSuccess)
+        else if (wait_for_device())
             cudaFreeAsync(p, d.stream);
-        else   // a capture or a failed context: the memory stays, since work may still read it
+        else   // a capture that forbids it or a failed context: the memory stays, since work may still read it
             cudaGetLastError();
     }
     if (other) cudaSetDevice(cur);
