@@ -963,6 +963,7 @@ int b200_destroy(b200_handle *h)
     cudaSetDevice(h->device);
     if (h->comp) cudaStreamSynchronize(h->comp);
     if (h->copy) cudaStreamSynchronize(h->copy);
+    DevRelease all;
     delete h;
     return B200_OK;
 }
@@ -2049,6 +2050,7 @@ int b200_group_destroy(b200_group *g)
     if (!g) return B200_EINVAL;
     cudaSetDevice(g->device);
     cudaStreamSynchronize(g->stream);
+    DevRelease all;
     delete g;
     return B200_OK;
 }

@@ -1,57 +1,61 @@
-// dev_pool.h -- the device memory of the handles, from a CUDA memory pool of the library's own per device.
+// dev_pool.h -- the device memory of the handles.
 //
 // A handle's buffers (for a 720p grid 14, some 900 MB with its tables) are mapped when it is made and unmapped
-// when it goes, at 0.1 to 0.6 ms a buffer: more than the work of the calls that make a handle for one pass
-// (the periodicity of one 720p frame: 4.5 of 7.5 ms). The pool keeps up to kPoolKeep bytes mapped for the
-// next handle and returns what is above that to the device at its next synchronization; when the device is out
-// of memory an allocation first returns all that is unused. The CUDA pool serves several threads and devices.
+// when it goes: more than the work of the calls that make a handle for one pass (the periodicity of one 720p
+// frame: 4.5 of 7.5 ms). So what a handle gives back stays mapped for the next one, at most 1 GiB a device:
+//
+//   up to kPoolBuffer bytes   a CUDA memory pool of the library's own, which keeps kPoolKeep bytes
+//   above                     buffers from cudaMalloc, of which kLargeKeep bytes are kept, the last released
+//
+// The line lies where the pool stops being the faster to map: new buffers of 1, 32, 64, 128 and 512 MiB take 0.23, 0.22,
+// 0.41, 0.81 and 3.2 ms from the pool, which maps 2 MiB at a time, and 0.36, 0.34, 0.34, 0.35 and 0.58 ms from cudaMalloc; their
+// release 0.20, 0.20, 0.40, 0.80 and 3.2 ms, and 0.30, 0.29, 0.30, 0.33 and 0.72 ms. Buffers that do not fit what is
+// kept (the spectra of a dense 1080p grid, 0.6 GB and more each) are mapped for every handle, as by cudaMalloc alone; a
+// large buffer is given out again only for one of its size or up to a fifth smaller, so handles of different
+// geometries that come and go in turn map again what 896 MiB do not hold for both (1 to 2 ms a change).
+// When the device is out of memory an allocation first returns all that is kept; release_memory() does so for others.
 //
 // The buffers are ready for, and freed after, every stream, as with cudaMalloc and cudaFree: an allocation
 // waits for its (empty) stream, a release first for the device (wait_for_device). The contents of a buffer are
-// undefined.
+// undefined. Any thread may call, with any device current.
 #pragma once
 
 #include <algorithm>
 #include <cstdint>
 #include <mutex>
-#include <unordered_set>
+#include <new>
+#include <unordered_map>
+#include <utility>
+#include <vector>
 
 #include <cuda_runtime.h>
 
 namespace b200 {
 
-constexpr uint64_t kPoolKeep = uint64_t(1) << 30;
-// Larger buffers come from cudaMalloc: the pool could not keep two of them, and maps them more slowly (the 3.6 GB
-// of spectra of a dense 1080p grid: a handle made in 27 ms from the pool, in 7 ms from cudaMalloc).
-constexpr size_t kPoolBuffer = size_t(512) << 20;
-
+constexpr uint64_t kPoolKeep = uint64_t(128) << 20;
+constexpr size_t kLargeKeep = size_t(896) << 20;
+constexpr size_t kPoolBuffer = size_t(32) << 20;
 constexpr size_t kWaitBuffer = 256;
 
 struct DevPool {
     cudaMemPool_t pool = nullptr;
     cudaStream_t stream = nullptr;   // orders the pool's allocations and releases; no work runs on it
     void *anchor = nullptr;          // keeps a block of small buffers mapped for wait_for_device
+    std::mutex mutex;                // of what follows
+    std::unordered_map<void *, size_t> held;            // large buffers in use, with their sizes
+    std::vector<std::pair<void *, size_t>> kept;        // and those kept, the oldest first
+    size_t kept_bytes = 0;
 };
 
-// the buffers above kPoolBuffer, so that a release knows them
-struct DirectBuffers {
-    std::mutex mutex;
-    std::unordered_set<void *> held;
-};
-inline DirectBuffers &direct_buffers()
-{
-    static DirectBuffers *d = new DirectBuffers;   // outlives every handle
-    return *d;
-}
-
-// the current device's pool (pool == nullptr: it has none), and the device's index
-inline cudaError_t device_pool(DevPool &out, int &dev)
+// the current device's pool (nullptr: it has none)
+inline cudaError_t device_pool(DevPool *&out)
 {
     static std::mutex mutex;
-    static DevPool pools[64];
+    static DevPool *pools[64] = {};   // outlive every handle
     static bool tried[64] = {};
+    out = nullptr;
+    int dev = 0;
     if (cudaError_t e = cudaGetDevice(&dev)) return e;
-    out = DevPool{};
     if (dev < 0 || dev >= 64) return cudaSuccess;
     std::lock_guard<std::mutex> lock(mutex);
     if (!tried[dev]) {
@@ -63,15 +67,16 @@ inline cudaError_t device_pool(DevPool &out, int &dev)
             props.location.type = cudaMemLocationTypeDevice;
             props.location.id = dev;
             uint64_t keep = kPoolKeep;
-            DevPool p;
-            if (cudaMemPoolCreate(&p.pool, &props) == cudaSuccess &&
-                cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess &&
-                cudaStreamCreateWithFlags(&p.stream, cudaStreamNonBlocking) == cudaSuccess) {
-                if (cudaMalloc(&p.anchor, kWaitBuffer) != cudaSuccess) cudaGetLastError();
+            DevPool *p = new DevPool;
+            if (cudaMemPoolCreate(&p->pool, &props) == cudaSuccess &&
+                cudaMemPoolSetAttribute(p->pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess &&
+                cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking) == cudaSuccess) {
+                if (cudaMalloc(&p->anchor, kWaitBuffer) != cudaSuccess) cudaGetLastError();
                 pools[dev] = p;
             } else {
                 cudaGetLastError();
-                if (p.pool) cudaMemPoolDestroy(p.pool);
+                if (p->pool) cudaMemPoolDestroy(p->pool);
+                delete p;
             }
         }
         tried[dev] = true;
@@ -91,39 +96,126 @@ inline bool wait_for_device()
     return cudaDeviceSynchronize() == cudaSuccess;
 }
 
+// what the current device's pool keeps unused goes back to the device
+inline cudaError_t release_memory()
+{
+    DevPool *d = nullptr;
+    if (cudaError_t e = device_pool(d)) return e;
+    if (!d) return cudaSuccess;
+    std::vector<std::pair<void *, size_t>> gone;
+    {
+        std::lock_guard<std::mutex> lock(d->mutex);
+        gone.swap(d->kept);
+        d->kept_bytes = 0;
+    }
+    cudaError_t err = cudaSuccess;
+    auto note = [&err](cudaError_t e) {
+        if (e && !err) err = e;
+    };
+    for (auto &b : gone) {
+        const cudaError_t e = cudaFree(b.first);
+        note(e);
+        if (e) {   // a capture that forbids it: for the next time
+            std::lock_guard<std::mutex> lock(d->mutex);
+            d->kept.push_back(b);
+            d->kept_bytes += b.second;
+        }
+    }
+    note(cudaStreamSynchronize(d->stream));   // the releases on it are then done
+    note(cudaMemPoolTrimTo(d->pool, 0));
+    return err;
+}
+
 // bytes of device memory on the current device, for every stream
 inline cudaError_t dev_alloc(void **p, size_t bytes)
 {
-    DevPool d;
-    int dev = 0;
-    if (cudaError_t e = device_pool(d, dev)) return e;
-    if (!d.pool) return cudaMalloc(p, bytes);
-    if (bytes > kPoolBuffer) {
-        cudaError_t e = cudaMalloc(p, bytes);
-        if (e == cudaErrorMemoryAllocation) {   // what the pool holds unused first
-            cudaGetLastError();
-            cudaMemPoolTrimTo(d.pool, 0);
-            e = cudaMalloc(p, bytes);
+    DevPool *d = nullptr;
+    if (cudaError_t e = device_pool(d)) return e;
+    if (!d) return cudaMalloc(p, bytes);
+    const bool large = bytes > kPoolBuffer;
+    if (large) {
+        bytes = (bytes + (size_t(2) << 20) - 1) >> 21 << 21;
+        std::lock_guard<std::mutex> lock(d->mutex);
+        auto best = d->kept.end();   // the smallest that is large enough, at most a quarter more
+        for (auto b = d->kept.begin(); b != d->kept.end(); ++b)
+            if (b->second >= bytes && b->second <= bytes + bytes / 4 && (best == d->kept.end() || b->second < best->second))
+                best = b;
+        if (best != d->kept.end()) {
+            *p = best->first;
+            d->held.insert(*best);
+            d->kept_bytes -= best->second;
+            d->kept.erase(best);
+            return cudaSuccess;
         }
-        if (e) return e;
-        DirectBuffers &b = direct_buffers();
-        std::lock_guard<std::mutex> lock(b.mutex);
-        b.held.insert(*p);
-        return cudaSuccess;
     }
-    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, d.pool, d.stream);
+    auto take = [&] { return large ? cudaMalloc(p, bytes) : cudaMallocFromPoolAsync(p, bytes, d->pool, d->stream); };
+    cudaError_t e = take();
     if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
-        cudaStreamSynchronize(d.stream);
-        cudaMemPoolTrimTo(d.pool, 0);
-        e = cudaMallocFromPoolAsync(p, bytes, d.pool, d.stream);
+        release_memory();
+        e = take();
     }
-    return e ? e : cudaStreamSynchronize(d.stream);
+    if (e) return e;
+    if (!large) return cudaStreamSynchronize(d->stream);
+    try {
+        std::lock_guard<std::mutex> lock(d->mutex);
+        d->held.emplace(*p, bytes);
+    } catch (const std::bad_alloc &) {
+        cudaFree(*p);
+        throw;
+    }
+    return cudaSuccess;
 }
 
+// While one lives, its thread's releases on the device that was current when it was made wait for the device once, at the first
+// of them: for a handle that goes, with nothing enqueued in between (720p, window 64: 185 us with a wait for
+// each of its buffers, 139 so).
+class DevRelease {
+public:
+    DevRelease() : outer_(current())
+    {
+        device_pool(pool_);
+        current() = this;
+    }
+    ~DevRelease()
+    {
+        current() = outer_;
+        if (small_) cudaStreamSynchronize(pool_->stream);
+    }
+    DevRelease(const DevRelease &) = delete;
+    DevRelease &operator=(const DevRelease &) = delete;
+
+    // a release to pool d: whether all work before it is done
+    static bool wait(DevPool *d)
+    {
+        DevRelease *r = current();
+        if (!r || r->pool_ != d) return wait_for_device();
+        return r->waited_ = r->waited_ || wait_for_device();
+    }
+    // a small buffer went to pool d's stream; what is above kPoolKeep goes back when that is synchronized
+    static void released(DevPool *d)
+    {
+        DevRelease *r = current();
+        if (r && r->pool_ == d)
+            r->small_ = true;
+        else
+            cudaStreamSynchronize(d->stream);
+    }
+
+private:
+    static DevRelease *&current()
+    {
+        static thread_local DevRelease *r = nullptr;
+        return r;
+    }
+    DevRelease *outer_;
+    DevPool *pool_ = nullptr;
+    bool waited_ = false, small_ = false;
+};
+
 // after all work of the memory's device
-inline void dev_free(void *p)
-{
+inline void dev_free(void *p) noexcept
+try {
     if (!p) return;
     cudaPointerAttributes at{};
     int cur = 0;
@@ -133,23 +225,42 @@ inline void dev_free(void *p)
     }
     const bool other = at.device != cur;
     if (other) cudaSetDevice(at.device);
-    DevPool d;
-    int dev = 0;
-    if (device_pool(d, dev) == cudaSuccess) {
-        bool direct = !d.pool;
-        if (!direct) {
-            DirectBuffers &b = direct_buffers();
-            std::lock_guard<std::mutex> lock(b.mutex);
-            direct = b.held.erase(p) > 0;
+    DevPool *d = nullptr;
+    const cudaError_t e = device_pool(d);
+    if (!e && !d) {
+        cudaFree(p);
+    } else if (e || !DevRelease::wait(d)) {
+        cudaGetLastError();   // a capture that forbids it or a failed context: the memory stays, since work may still read it
+    } else {
+        std::vector<std::pair<void *, size_t>> gone;   // given back outside the lock
+        bool large = false;
+        {
+            std::lock_guard<std::mutex> lock(d->mutex);
+            const auto b = d->held.find(p);
+            large = b != d->held.end();
+            if (large) {
+                const std::pair<void *, size_t> buffer = *b;
+                d->held.erase(b);
+                size_t drop = 0;
+                if (buffer.second > kLargeKeep) {
+                    gone.push_back(buffer);
+                } else {
+                    while (d->kept_bytes + buffer.second > kLargeKeep) d->kept_bytes -= d->kept[drop++].second;
+                    gone.assign(d->kept.begin(), d->kept.begin() + drop);
+                    d->kept.erase(d->kept.begin(), d->kept.begin() + drop);
+                    d->kept.push_back(buffer);
+                    d->kept_bytes += buffer.second;
+                }
+            }
         }
-        if (direct)
-            cudaFree(p);
-        else if (wait_for_device())
-            cudaFreeAsync(p, d.stream);
-        else   // a capture that forbids it or a failed context: the memory stays, since work may still read it
-            cudaGetLastError();
+        for (auto &b : gone) cudaFree(b.first);
+        if (!large) {
+            cudaFreeAsync(p, d->stream);
+            DevRelease::released(d);
+        }
     }
     if (other) cudaSetDevice(cur);
+} catch (const std::bad_alloc &) {   // no room for the lists: the memory stays
 }
 
 }   // namespace b200

@@ -488,6 +488,7 @@ int b200_stab_create(int height, int width, const uint8_t *text, int size, int d
 
 int b200_stab_destroy(b200_stab *s)
 {
+    b200::DevRelease all;
     delete s;
     return B200_OK;
 }
