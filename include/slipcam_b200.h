@@ -82,8 +82,16 @@ typedef struct b200_handle b200_handle;
  * as chosen by bindings.cpp:38-44. On failure *out is NULL and b200_last_error(NULL) says why. */
 B200_API int b200_create(const b200_params *p, int device, b200_handle **out);
 
-/* Free the handle and its device memory (the Correlator's destructor, cxx/framecor.h:48). */
+/* Free the handle (the Correlator's destructor, cxx/framecor.h:48). Its device memory is kept for the next
+ * handle of the process, up to 1 GiB a device in all; what is above that goes back to the device
+ * now. No work on the handle may be enqueued meanwhile; work that is is waited for. */
 B200_API int b200_destroy(b200_handle *h);
+
+/* Give the device memory kept of destroyed handles (b200_destroy, b200_stab_destroy, b200_group_destroy)
+ * back to the device, for a program that wants it elsewhere; handles in use are not touched. The
+ * library does so itself when an allocation of its own finds the device full. B200_ERUNTIME if there
+ * is no such device, or during a capture that forbids cudaFree. No counterpart in the reference. */
+B200_API int b200_release_memory(int device);
 
 /* The last error message of a handle, or of the calling thread's last b200_create if h is NULL. */
 B200_API const char *b200_last_error(const b200_handle *h);

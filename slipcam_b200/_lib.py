@@ -29,6 +29,7 @@ _vp, _i, _u8p = ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p
 SIGNATURES = {
     'b200_create': (_i, [ctypes.POINTER(Params), _i, ctypes.POINTER(_vp)]),
     'b200_destroy': (_i, [_vp]),
+    'b200_release_memory': (_i, [_i]),
     'b200_last_error': (ctypes.c_char_p, [_vp]),
     'b200_set_reference': (_i, [_vp, _u8p]),
     'b200_correlate': (_i, [_vp, _u8p, _i, _vp, _i, _vp, _vp, _vp, _vp]),

@@ -968,6 +968,19 @@ int b200_destroy(b200_handle *h)
     return B200_OK;
 }
 
+int b200_release_memory(int device)
+{
+    int cur = 0;
+    if (cudaGetDevice(&cur) != cudaSuccess || cudaSetDevice(device) != cudaSuccess) {
+        cudaGetLastError();
+        return B200_ERUNTIME;
+    }
+    const cudaError_t e = release_memory();
+    if (e) cudaGetLastError();
+    cudaSetDevice(cur);
+    return e ? B200_ERUNTIME : B200_OK;
+}
+
 const char *b200_last_error(const b200_handle *h) { return h ? h->err.c_str() : g_create_error.c_str(); }
 
 int b200_set_form(b200_handle *h, int form)

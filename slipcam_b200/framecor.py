@@ -255,6 +255,13 @@ class Correlator:
         return out
 
 
+def release_memory(device=0):
+    """Give the device memory that destroyed correlators left mapped for the next ones (at most 1 GiB) back to
+    the device, for other allocators; correlators in use are not touched."""
+    if _lib.lib().b200_release_memory(int(device)) != _lib.OK:
+        raise RuntimeError(f'framecor: the memory of device {device} could not be released')
+
+
 def sat(frames):
     """The summed-area tables of uint8 CUDA frames (n, h, w): (sat uint32 as int64 tensor,
     sat2 int64), each (n, h + 1, w + 1); the first row and column are zero."""
