@@ -51,10 +51,11 @@ extern "C" {
 
 /* the arithmetic of the transforms */
 #define B200_FORM_AUTO 0   /* the library's choice, and the default: B200_FORM_TC for windows above 32 px
-                              where it holds the geometry (FFT size up to 160, search up to 63 px),
-                              else B200_FORM_FFT32 */
+                              where it takes the geometry, else B200_FORM_FFT32 */
 #define B200_FORM_FFT32 1  /* FP32 FFTs on the CUDA cores */
-#define B200_FORM_TC 2     /* DFT-matrix GEMMs on the tensor cores, FP16 operands, FP32 accumulation */
+#define B200_FORM_TC 2     /* DFT-matrix GEMMs on the tensor cores, FP16 operands, FP32 accumulation: FFT sizes
+                              up to 160 (window + 2 search, rounded up to 16, 32, 48, 64, 80, 96, 128, 144 or
+                              160), searches up to 37 px at 80, 44 at 96, 48 at 128, 49 at 144 and 54 at 160 */
 #define B200_FORM_I8 3     /* direct correlation on the tensor cores in exact integers (uint8 x uint8,
                               int32 accumulation), normalized after: windows up to 181 px, search
                               windows (window + 2 search) up to 256 px */

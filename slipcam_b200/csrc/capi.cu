@@ -371,36 +371,13 @@ void launch_corr_i8(const CorrArgs &a, const uint8_t *refwin, const int *sref, i
         corr_i8_kernel<false><<<unsigned(grid), kI8Threads, g.smem, s>>>(x);
 }
 
-// The geometries the tensor-core form takes, by FFT size and surface side: those whose box of variance
-// denominators (rows of M + 3 floats rounded up to 4) fits the larger of its chip and S5 operands, with
-// NO columns of correlation beside 512 - NO of other accumulators. The kernel itself holds every M up to
-// 128; the others stay on the FP32 form, whose accuracy their callers have.
-template <int N>
-bool tc_fits_n(int M)
+// The largest search the tensor-core form takes at each FFT size, 0 where it has no kernel. The kernel itself holds
+// surfaces of up to 128 shifts a side, 63 px of search; the line lies lower because of the precision: beyond it the form's
+// FP16 operands (2e-3 on a surface value, 1e-4 relative on the SNR) would take the place of FP32's 1e-5 in
+// geometries whose callers have had that. Up to 64 every search that the FFT size leaves room for is below it.
+constexpr int tc_max_search(int N)
 {
-    constexpr int KP = TcGeo<N>::KP, T1 = (N + 127) / 128;
-    constexpr size_t room = std::max<size_t>(size_t(N) * N * 2, size_t(16) * (2 * KP) * 16);
-    const int NO = (M + 15) / 16 * 16;
-    const int used = std::max({2 * KP * T1, 2 * N, 2 * NO});
-    return size_t((M + 3 + 3) / 4 * 4) * M * 4 <= room && used + NO <= 512;
-}
-
-// whether the tensor-core kernel holds this geometry: FFT size up to 160, up to 128 shifts per axis
-bool tc_fits(int N, int M)
-{
-    if (M > 128) return false;
-    switch (N) {
-    case 16: return tc_fits_n<16>(M);
-    case 32: return tc_fits_n<32>(M);
-    case 48: return tc_fits_n<48>(M);
-    case 64: return tc_fits_n<64>(M);
-    case 80: return tc_fits_n<80>(M);
-    case 96: return tc_fits_n<96>(M);
-    case 128: return tc_fits_n<128>(M);
-    case 144: return tc_fits_n<144>(M);
-    case 160: return tc_fits_n<160>(M);
-    default: return false;
-    }
+    return N == 16 ? 20 : N == 32 || N == 48 ? 30 : N == 64 || N == 80 ? 37 : N == 96 ? 44 : N == 128 ? 48 : N == 144 ? 49 : N == 160 ? 54 : 0;
 }
 
 #define B200_DISPATCH_TC(N_, F, ...)                                                               \
@@ -928,7 +905,7 @@ int b200_create(const b200_params *p, int device, b200_handle **out)
         h->d_ref.alloc(size_t(h->height) * h->fpitch);
         h->d_status.alloc(1);
         CK(cudaMemset(h->d_status.p, 0, sizeof(int)));
-        h->tc_ok = tc_fits(N, h->M);
+        h->tc_ok = h->R <= tc_max_search(N);
         if (h->tc_ok) {
             std::vector<uint16_t> dt(size_t(tc_rt(N)) * N);
             tc_dft_table(N, dt.data());
@@ -988,9 +965,12 @@ int b200_set_form(b200_handle *h, int form)
     return guarded(h, [&] {
         if (form != B200_FORM_AUTO && form != B200_FORM_FFT32 && form != B200_FORM_TC && form != B200_FORM_I8)
             fail(B200_EINVAL, "unknown form " + std::to_string(form));
-        if (form == B200_FORM_TC && !h->tc_ok)
-            fail(B200_EINVAL, "the tensor-core form holds FFT sizes up to 160 and search ranges up to 63 px, not "
-                                  + std::to_string(h->N) + " and " + std::to_string(h->R));
+        if (form == B200_FORM_TC && !h->tc_ok) {
+            if (!tc_max_search(h->N))
+                fail(B200_EINVAL, "the tensor-core form holds FFT sizes up to 160, not " + std::to_string(h->N));
+            fail(B200_EINVAL, "the tensor-core form takes searches up to " + std::to_string(tc_max_search(h->N))
+                                  + " px at FFT size " + std::to_string(h->N) + ", not " + std::to_string(h->R));
+        }
         if (form == B200_FORM_I8 && !h->i8_ok)
             fail(B200_EINVAL, "the exact tensor-core form holds windows up to " + std::to_string(kI8MaxWindow)
                                   + " px and search windows up to 256 px, not " + std::to_string(h->W) + " and "
