@@ -1154,8 +1154,8 @@ int b200_correlate_device_surfaces(b200_handle *h, const uint8_t *frames, int n,
 // held until the process exits, instead of in buffers of the handle. Nothing here calls cudaMalloc,
 // cudaFree or any allocating routine.
 //
-// The array holds 32 MiB: the tables of one 1920 x 1080 frame (16.0 bytes per pixel). Frames are
-// correlated as many per launch as their tables fit. In host code the array's name is only a
+// The array holds 32 MiB: the room of one 1920 x 1080 frame (16 bytes per pixel, 12 of which its tables use). Frames are
+// correlated as many per launch as have room. In host code the array's name is only a
 // stand-in for its device address, so the address is looked up with cudaGetSymbolAddress, once per
 // device, by the first call on that device with the device current; make that first call before
 // any stream capture. Every call on a device shares the array, so calls that overlap on the GPU
@@ -1186,13 +1186,14 @@ int b200_correlate_device_noalloc(b200_handle *h, const uint8_t *frames, int n, 
         if (n == 0) return;
         if (!frames || pitch < h->width || !offset || !peak || !snr || !cov)
             fail(B200_EINVAL, "null input or output, or a pitch below the width");
-        // the room for one frame: two summed-area tables (8 bytes an entry for the squares), variance denominators
+        // the room set aside for one frame: two summed-area tables, variance denominators. The table of squares has 8
+        // bytes an entry, of which it uses 4: the largest frame taken and the frames per launch stay as callers know them
         const size_t b32 = size_t(h->sat_size()) * sizeof(uint32_t), b64 = size_t(h->sat_size()) * sizeof(int64_t);
         const size_t bd = size_t(h->dinv_size()) * sizeof(float);
         const size_t per_frame = align256(b32) + align256(b64) + align256(bd);
         if (per_frame > kNoAllocBytes)
-            fail(B200_EINVAL, "the frame is too large for the no-allocation entry point: its tables need "
-                                  + std::to_string(per_frame) + " bytes, the static scratch holds "
+            fail(B200_EINVAL, "the frame is too large for the no-allocation entry point, which sets aside "
+                                  + std::to_string(per_frame) + " bytes for one of its size and holds "
                                   + std::to_string(kNoAllocBytes) + " (one 1920 x 1080 frame)");
         if (h->device < 0 || h->device >= 64) fail(B200_EINVAL, "device index out of range");
         CK(cudaSetDevice(h->device));
