@@ -573,7 +573,7 @@ struct b200_handle {
         CorrArgs a = corr_args(frames, pitch, nf, gross, gross_mode, sat, dinv, offset, peak, snr, cov, surface);
         a.bstat = bstat;
         a.peaks = refine ? peaks : nullptr;
-        run_corr_tail(a, nf, dinv, arith, s);
+        run_corr(a, nf, arith, s);
         if (refine) {
             CK(cudaMemsetAsync(queue, 0, sizeof(int), s));
             static bool attr[64] = {};
@@ -620,15 +620,6 @@ struct b200_handle {
         launch_dinv(sat, sat2, nf, height, width, W, dinv, dinv_size(), dpitch(), bstat, s);
     }
 
-    // the correlation of nf frames with their tables at sat / dinv, in the form `arith`
-    void run_corr(const uint8_t *frames, int pitch, int nf, const int32_t *gross, int gross_mode, const uint32_t *sat,
-                  const float *dinv, float *offset, float *peak, float *snr, float *cov, float *surface, int arith,
-                  cudaStream_t s)
-    {
-        const CorrArgs a = corr_args(frames, pitch, nf, gross, gross_mode, sat, dinv, offset, peak, snr, cov, surface);
-        run_corr_tail(a, nf, dinv, arith, s);
-    }
-
     // the arguments of the correlation kernels for nf frames with their tables at sat / dinv
     CorrArgs corr_args(const uint8_t *frames, int pitch, int nf, const int32_t *gross, int gross_mode,
                        const uint32_t *sat, const float *dinv, float *offset, float *peak, float *snr, float *cov,
@@ -669,8 +660,8 @@ struct b200_handle {
         return a;
     }
 
-    // the launch of run_corr (and its profiling events)
-    void run_corr_tail(const CorrArgs &a, int nf, const float *dinv, int arith, cudaStream_t s)
+    // the launch of the correlation in the form `arith` (and its profiling events)
+    void run_corr(const CorrArgs &a, int nf, int arith, cudaStream_t s)
     {
         Timed t{};
         if (profiling) {
@@ -1598,7 +1589,7 @@ int b200_coarse_track_device(b200_handle *h, const uint8_t *frames, int n, int p
                     CK(cudaGetLastError());
                     h->launches += 1;
                 } else {
-                    h->run_corr_tail(a, 1, a.dinv, B200_FORM_FFT32, s);   // counts its launch
+                    h->run_corr(a, 1, B200_FORM_FFT32, s);   // counts its launch
                     CK(launch_ncc_peaks(surf, int(nwin), h->M, h->d_cpeaks.p, s));
                     h->launches += 1;
                 }

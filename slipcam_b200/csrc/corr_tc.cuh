@@ -144,13 +144,6 @@ __device__ __forceinline__ float ldg_here(const float *p)
     return v;
 }
 
-__device__ __forceinline__ float4 ldg_here(const float4 *p)
-{
-    float4 v;
-    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
-    return v;
-}
-
 __device__ __forceinline__ uint4 ldg_here(const uint4 *p)
 {
     uint4 v;
@@ -693,7 +686,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) corr_tc_kernel(const __grid_con
     } else if (warp == kTcFetch) {
         // ---- the reference spectrum of the pairs, chunk after chunk
         if (lane == 0) {
-            uint32_t g = 0;   // chunks so far: slot g % 4, its use g / 4
+            uint32_t g = 0;   // chunks so far: slot g % kTcSlots, its use g / kTcSlots
             for (uint32_t n = 0;; ++n) {
                 const PairSetup &e = ring[n & 3];
                 if (!tc_entry_one(e, n, ab) || e.end) break;
@@ -729,7 +722,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) corr_tc_kernel(const __grid_con
 #pragma unroll 1
                 for (int c = 16 * part; c < N; c += 16 * kTcParts) {
                     float y[16];
-                    tc::tmem_ld_cols<16>(tl + col + uint32_t(c), y);
+                    tc::tmem_ld16(tl + col + uint32_t(c), y);
                     if (im && kap == 0) {   // the Nyquist row is not S's row 0
 #pragma unroll
                         for (int t = 0; t < 16; ++t) y[t] = 0.0f;

@@ -156,19 +156,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16])
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// 32 consecutive columns, without waiting (several loads may be issued before tmem_wait)
-__device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, uint32_t (&r)[32])
-{
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-        "%15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr));
-}
-
+// the same without waiting (several loads may be issued before tmem_wait)
 __device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, uint32_t *r)
 {
     asm volatile(
@@ -195,20 +183,6 @@ __device__ __forceinline__ void tmem_ld8_nowait(uint32_t taddr, uint32_t (&r)[8]
 
 __device__ __forceinline__ void tmem_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// NC (a multiple of 16) consecutive columns of this thread's lane into v, one wait for all
-template <int NC>
-__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, float (&v)[NC])
-{
-    static_assert(NC % 16 == 0, "16-column granules");
-    uint32_t r[NC];
-#pragma unroll
-    for (int c = 0; c + 32 <= NC; c += 32) tmem_ld32_nowait(taddr + uint32_t(c), *reinterpret_cast<uint32_t(*)[32]>(r + c));
-    if constexpr (NC % 32) tmem_ld16_nowait(taddr + uint32_t(NC - 16), r + NC - 16);
-    tmem_wait();
-#pragma unroll
-    for (int c = 0; c < NC; ++c) v[c] = __uint_as_float(r[c]);
-}
-
 // the mbarrier expects `bytes` more bytes of asynchronous copies in the current phase (one arrival)
 __device__ __forceinline__ void mbar_expect_tx(uint64_t *mbar, uint32_t bytes)
 {
@@ -224,14 +198,6 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t b
                  "l"(src), "r"(bytes), "r"(smem_u32(mbar))
                  : "memory");
 }
-
-// 4-byte asynchronous copies global -> shared, completed by cp_async_wait_all
-__device__ __forceinline__ void cp_async4(void *dst, const void *src)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 #endif   // __CUDACC__
 
