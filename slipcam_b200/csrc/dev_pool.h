@@ -4,7 +4,7 @@
 // when it goes: more than the work of the calls that make a handle for one pass (the periodicity of one 720p
 // frame: 4.5 of 7.5 ms). So what a handle gives back stays mapped for the next one, at most 1 GiB a device:
 //
-//   up to kPoolBuffer bytes   a CUDA memory pool of the library's own, which keeps kPoolKeep bytes
+//   up to kPoolBuffer bytes   a CUDA memory pool of the library's own, which keeps what the others leave of kKeep
 //   above                     buffers from cudaMalloc, of which kLargeKeep bytes are kept, the last released
 //
 // The line lies where the pool stops being the faster to map: new buffers of 1, 32, 64, 128 and 512 MiB take 0.23, 0.22,
@@ -12,7 +12,7 @@
 // release 0.20, 0.20, 0.40, 0.80 and 3.2 ms, and 0.30, 0.29, 0.30, 0.33 and 0.72 ms. Buffers that do not fit what is
 // kept (the spectra of a dense 1080p grid, 0.6 GB and more each) are mapped for every handle, as by cudaMalloc alone; a
 // large buffer is given out again only for one of its size or up to a fifth smaller, so handles of different
-// geometries that come and go in turn map again what 896 MiB do not hold for both (1 to 2 ms a change).
+// geometries that come and go in turn map again what 1 GiB does not hold for both (1 to 2 ms a change).
 // When the device is out of memory an allocation first returns all that is kept; release_memory() does so for others.
 //
 // The buffers are ready for, and freed after, every stream, as with cudaMalloc and cudaFree: an allocation
@@ -32,7 +32,7 @@
 
 namespace b200 {
 
-constexpr uint64_t kPoolKeep = uint64_t(128) << 20;
+constexpr size_t kKeep = size_t(1) << 30;
 constexpr size_t kLargeKeep = size_t(896) << 20;
 constexpr size_t kPoolBuffer = size_t(32) << 20;
 constexpr size_t kWaitBuffer = 256;
@@ -45,6 +45,13 @@ struct DevPool {
     std::unordered_map<void *, size_t> held;            // large buffers in use, with their sizes
     std::vector<std::pair<void *, size_t>> kept;        // and those kept, the oldest first
     size_t kept_bytes = 0;
+
+    // the pool's share of kKeep (its own rule counts the buffers in use too); call when kept_bytes has changed
+    cudaError_t share() const
+    {
+        uint64_t keep = kKeep - kept_bytes;
+        return cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    }
 };
 
 // the current device's pool (nullptr: it has none)
@@ -66,10 +73,8 @@ inline cudaError_t device_pool(DevPool *&out)
             props.handleTypes = cudaMemHandleTypeNone;
             props.location.type = cudaMemLocationTypeDevice;
             props.location.id = dev;
-            uint64_t keep = kPoolKeep;
             DevPool *p = new DevPool;
-            if (cudaMemPoolCreate(&p->pool, &props) == cudaSuccess &&
-                cudaMemPoolSetAttribute(p->pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess &&
+            if (cudaMemPoolCreate(&p->pool, &props) == cudaSuccess && p->share() == cudaSuccess &&
                 cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking) == cudaSuccess) {
                 if (cudaMalloc(&p->anchor, kWaitBuffer) != cudaSuccess) cudaGetLastError();
                 pools[dev] = p;
@@ -107,6 +112,7 @@ inline cudaError_t release_memory()
         std::lock_guard<std::mutex> lock(d->mutex);
         gone.swap(d->kept);
         d->kept_bytes = 0;
+        d->share();
     }
     cudaError_t err = cudaSuccess;
     auto note = [&err](cudaError_t e) {
@@ -119,6 +125,7 @@ inline cudaError_t release_memory()
             std::lock_guard<std::mutex> lock(d->mutex);
             d->kept.push_back(b);
             d->kept_bytes += b.second;
+            d->share();
         }
     }
     note(cudaStreamSynchronize(d->stream));   // the releases on it are then done
@@ -145,6 +152,7 @@ inline cudaError_t dev_alloc(void **p, size_t bytes)
             d->held.insert(*best);
             d->kept_bytes -= best->second;
             d->kept.erase(best);
+            d->share();
             return cudaSuccess;
         }
     }
@@ -180,7 +188,7 @@ public:
     ~DevRelease()
     {
         current() = outer_;
-        if (small_) cudaStreamSynchronize(pool_->stream);
+        if (sync_) cudaStreamSynchronize(pool_->stream);
     }
     DevRelease(const DevRelease &) = delete;
     DevRelease &operator=(const DevRelease &) = delete;
@@ -192,12 +200,12 @@ public:
         if (!r || r->pool_ != d) return wait_for_device();
         return r->waited_ = r->waited_ || wait_for_device();
     }
-    // a small buffer went to pool d's stream; what is above kPoolKeep goes back when that is synchronized
+    // a buffer went back, or the pool's share is smaller: what is above that goes when its stream is synchronized
     static void released(DevPool *d)
     {
         DevRelease *r = current();
         if (r && r->pool_ == d)
-            r->small_ = true;
+            r->sync_ = true;
         else
             cudaStreamSynchronize(d->stream);
     }
@@ -210,7 +218,7 @@ private:
     }
     DevRelease *outer_;
     DevPool *pool_ = nullptr;
-    bool waited_ = false, small_ = false;
+    bool waited_ = false, sync_ = false;
 };
 
 // after all work of the memory's device
@@ -250,14 +258,13 @@ try {
                     d->kept.erase(d->kept.begin(), d->kept.begin() + drop);
                     d->kept.push_back(buffer);
                     d->kept_bytes += buffer.second;
+                    d->share();
                 }
             }
         }
         for (auto &b : gone) cudaFree(b.first);
-        if (!large) {
-            cudaFreeAsync(p, d->stream);
-            DevRelease::released(d);
-        }
+        if (!large) cudaFreeAsync(p, d->stream);
+        DevRelease::released(d);
     }
     if (other) cudaSetDevice(cur);
 } catch (const std::bad_alloc &) {   // no room for the lists: the memory stays

@@ -12,7 +12,7 @@ CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
 RUNTIME = r'''
 #pragma once
 // A device of `capacity` bytes. Buffers are host addresses that are never used again. Releases on the pool's stream
-// come about when it is synchronized; the pool then returns what is unused above its threshold.
+// come about when it is synchronized; the pool then returns what is unused while it holds more than its threshold.
 #include <cstddef>
 #include <cstdint>
 #include <cstdlib>
@@ -29,7 +29,12 @@ struct Fake {
     int mallocs = 0, waits = 0, pool_new = 0, device_syncs = 0;
     bool forbid = false, pools = true;
     size_t mapped() const { return direct + pooled; }
-    void trim(size_t keep) { if (unused > keep) { pooled -= unused - keep; unused = keep; } }
+    void trim(size_t keep)
+    {
+        const size_t n = pooled > keep ? (unused < pooled - keep ? unused : pooled - keep) : 0;
+        pooled -= n;
+        unused -= n;
+    }
 };
 inline Fake &fake() { static Fake f; return f; }
 struct cudaMemPoolProps { int allocType, handleTypes; struct { int type, id; } location; };
@@ -139,6 +144,16 @@ int main(int, char **argv)
         void *a = get(100 * MB);
         CHECK(f.mallocs == 3);
         dev_free(a);
+        release_memory();
+        f.pool_new = 0;   // small handles side by side, again and again: their buffers stay, whatever is in use
+        for (int i = 0; i < 4; ++i) {
+            void *s[4][3];
+            for (auto &h : s)
+                for (void *&p : h) p = get(30 * MB);
+            for (auto &h : s)
+                for (void *p : h) dev_free(p);
+        }
+        CHECK(f.pool_new <= 12);
     } else if (test("bound")) {   // at most 1 GiB stays, also of buffers that are each well below it, at once
         for (size_t n : {1 * MB, 30 * MB, 60 * MB, 250 * MB, 900 * MB}) {
             std::vector<void *> p;
