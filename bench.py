@@ -63,7 +63,6 @@ def tc_flops(n, m):
     return 3 * 4 * 128 * n * n + 4 * 128 * no * kp
 
 
-
 class Clocks:
     """nvidia-smi samples of one GPU while running."""
     FIELDS = ('index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,'
@@ -112,15 +111,16 @@ class Clocks:
 
 # dram bytes per 16-frame launch of the correlation kernel (dram__bytes_read.sum + dram__bytes_write.sum
 # of one ncu capture of this workload's launch, per form)
-TRAFFIC_PER_LAUNCH = {("fft32", 160): 328990464, ("tc", 160): 380023808}
+TRAFFIC_PER_LAUNCH = {("fft32", 160): 330064384, ("tc", 160): 581009920}
 
 
 def dft_gemm_flops(n, m):
-    """useful DFT-GEMM work of one window (FFT size n, m shifts per axis), one pass at the GEMM form's
-    operand sizes: forward row real DFT 4 n^2 (n/2+1) + column complex DFT 8 n^2 (n/2+1); inverse pruned to the m
-    output rows and columns, column 8 m n (n/2+1) + row 4 m^2 (n/2+1) (38.0 MFLOP at n = 160, m = 97)"""
+    """useful DFT-GEMM work of one window (FFT size n, m shifts per axis), one pass at the GEMM form's operand sizes,
+    nh = n/2 + 1: forward row real DFT 4 n^2 nh; column complex DFT 4 n^2 nh (columns r < n/2 of the DFT matrices give
+    the frequencies r and n - r); inverse column the same, 8 n nh min(m, n/2), pruned to the m output rows; inverse row 4 m^2 nh
+    (27.9 MFLOP at n = 160, m = 97)"""
     nh = n // 2 + 1
-    return 4 * n * n * nh + 8 * n * n * nh + 8 * m * n * nh + 4 * m * m * nh
+    return 4 * n * n * nh + 4 * n * n * nh + 8 * n * nh * min(m, n // 2) + 4 * m * m * nh
 
 
 def direct_ops(w, m):
@@ -459,8 +459,8 @@ def run_b200(args):
                                            f' (profiles/corr_{args.form}_720p_w64_s48.md)' if traffic else None,
                          'kernel': kname, 'kernel_ms_per_launch': kernel_ms / max(kernel_launches, 1),
                          'peak_source': peak_src, 'work_per_window': work, 'executed_per_window': executed,
-                         'work_source': {'tc': 'useful DFT-GEMM FLOPs, one pass (forward 4n^2 nh + 8n^2 nh, '
-                                                'inverse 8 m n nh + 4 m^2 nh)',
+                         'work_source': {'tc': 'useful DFT-GEMM FLOPs, one pass (forward 4n^2 nh + 4n^2 nh, '
+                                                'inverse 8 n nh min(m, n/2) + 4 m^2 nh)',
                                          'int8': 'useful integer ops of the direct correlation, 2 W^2 M^2',
                                          'fft32': 'useful FFT FLOPs 2 x 2.5 n^2 log2 n^2 + 6 n nh'}[args.form],
                          'useful_fft_flop_per_window': fft_flops(fft_n)},

@@ -36,12 +36,13 @@
 // (stores of operands, copies, loads through L1) all but waits while MMAs run: S2 starts when both halves
 // of its operand are in.
 //
-// Measured at 720p, window 64, search 48 (N = 160, 39,200 pairs a launch): 2.16 ms, 15,500 cycles a pair
+// Measured at 720p, window 64, search 48 (N = 160, 39,200 pairs a launch): 2.20 ms, 16,300 cycles a pair
 // and SM, where one role after the other in the same 12 warps took 3.96 ms; N = 96 (window 48, search 24)
-// 10,600 cycles. The MMAs are 5,500 of them. What bounds a pair is the instruction cache: the roles' code,
-// each executed once a pair, comes at 10 to 16 cycles an instruction (more warps on the same code helped,
-// unrolled copies of it hurt: 179 KB of code took 2.39 ms, rolled into 68 KB the same design 2.16 ms),
-// and the chain S4, Q's drain, S5, Yi, its drain, S2, S3 with the epilogue's hold on c beside it.
+// 10,600 cycles. The MMAs are 5,500 of them. No unit is full: ncu of such a launch has the tensor pipe 37 % busy, the
+// issue slots 50 %, the L1 and shared memory 49 %. Of 15.9 stalled warps per issue 5.2 wait at a barrier and 4.4 for TMEM
+// or L2 loads: what bounds a pair is the chain S4, Q's drain, S5, Yi, its drain, S2, S3 with the
+// epilogue's hold on c beside it. The code has to stay small: unrolled to 179 KB the same design took 2.39 ms
+// against 2.16 in 68 KB, and in the latter only 0.3 of those stalls are for instructions.
 //
 // TMEM columns: Q [0, 2N), then c [0, NO) and Yi [NO, NO + N) once it is drained; Yr [2N, 3N); S2's
 // products replace Y where it was.
@@ -197,8 +198,8 @@ struct TcBars {
 };
 
 // wait for the phase `parity` of the mbarrier; false if another role gave up or two seconds went by
-// (the abort flag is then set for the others). The polling is one function for all roles: what they
-// execute has to fit the SM's instruction cache together.
+// (the abort flag is then set for the others). The polling is one function for all roles, for the size of the
+// code.
 __device__ __noinline__ bool tc_wait_poll(uint64_t *bar, uint32_t parity, volatile int *abort)
 {
     uint64_t t0, t1;
