@@ -4,8 +4,12 @@
 // when it goes: more than the work of the calls that make a handle for one pass (the periodicity of one 720p
 // frame: 4.5 of 7.5 ms). So what a handle gives back stays mapped for the next one, at most 1 GiB a device:
 //
-//   up to kPoolBuffer bytes   a CUDA memory pool of the library's own, which keeps what the others leave of kKeep
+//   up to kPoolBuffer bytes   a CUDA memory pool of the library's own
 //   above                     buffers from cudaMalloc, of which kLargeKeep bytes are kept, the last released
+//
+// What the pool has unused and the large buffers kept are kKeep bytes at most together; where they would be more, what was
+// used last stays: a release of small buffers drops the oldest of the kept, one that keeps a large buffer what the
+// pool has too much (balance).
 //
 // The line lies where the pool stops being the faster to map: new buffers of 1, 32, 64, 128 and 512 MiB take 0.23, 0.22,
 // 0.41, 0.81 and 3.2 ms from the pool, which maps 2 MiB at a time, and 0.36, 0.34, 0.34, 0.35 and 0.58 ms from cudaMalloc; their
@@ -46,11 +50,35 @@ struct DevPool {
     std::vector<std::pair<void *, size_t>> kept;        // and those kept, the oldest first
     size_t kept_bytes = 0;
 
-    // the pool's share of kKeep (its own rule counts the buffers in use too); call when kept_bytes has changed
-    cudaError_t share() const
+    // The bound, after releases: of small buffers alone, or with large ones kept. (The pool's own threshold is no use for
+    // it: it counts the buffers in use, and a few handles alive would have every release unmap memory.)
+    void balance(bool large)
     {
-        uint64_t keep = kKeep - kept_bytes;
-        return cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        cudaStreamSynchronize(stream);   // the releases on it are then done
+        uint64_t used = 0, reserved = 0;
+        if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess ||
+            cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess) {
+            cudaGetLastError();
+            return;
+        }
+        const size_t idle = reserved > used ? size_t(reserved - used) : 0;
+        std::vector<std::pair<void *, size_t>> gone;
+        size_t share = 0;
+        {
+            std::lock_guard<std::mutex> lock(mutex);
+            if (!large) drop(idle < kKeep ? kKeep - idle : 0, gone);
+            share = kKeep - kept_bytes;
+        }
+        for (auto &b : gone) cudaFree(b.first);
+        if (idle > share) cudaMemPoolTrimTo(pool, size_t(used) + share);
+    }
+    // the oldest of the kept into gone, down to `most` bytes; under the lock
+    void drop(size_t most, std::vector<std::pair<void *, size_t>> &gone)
+    {
+        size_t n = 0;
+        while (kept_bytes > most) kept_bytes -= kept[n++].second;
+        gone.insert(gone.end(), kept.begin(), kept.begin() + n);
+        kept.erase(kept.begin(), kept.begin() + n);
     }
 };
 
@@ -74,7 +102,9 @@ inline cudaError_t device_pool(DevPool *&out)
             props.location.type = cudaMemLocationTypeDevice;
             props.location.id = dev;
             DevPool *p = new DevPool;
-            if (cudaMemPoolCreate(&p->pool, &props) == cudaSuccess && p->share() == cudaSuccess &&
+            uint64_t all = UINT64_MAX;   // balance() returns what is too much
+            if (cudaMemPoolCreate(&p->pool, &props) == cudaSuccess &&
+                cudaMemPoolSetAttribute(p->pool, cudaMemPoolAttrReleaseThreshold, &all) == cudaSuccess &&
                 cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking) == cudaSuccess) {
                 if (cudaMalloc(&p->anchor, kWaitBuffer) != cudaSuccess) cudaGetLastError();
                 pools[dev] = p;
@@ -112,7 +142,6 @@ inline cudaError_t release_memory()
         std::lock_guard<std::mutex> lock(d->mutex);
         gone.swap(d->kept);
         d->kept_bytes = 0;
-        d->share();
     }
     cudaError_t err = cudaSuccess;
     auto note = [&err](cudaError_t e) {
@@ -125,7 +154,6 @@ inline cudaError_t release_memory()
             std::lock_guard<std::mutex> lock(d->mutex);
             d->kept.push_back(b);
             d->kept_bytes += b.second;
-            d->share();
         }
     }
     note(cudaStreamSynchronize(d->stream));   // the releases on it are then done
@@ -152,7 +180,6 @@ inline cudaError_t dev_alloc(void **p, size_t bytes)
             d->held.insert(*best);
             d->kept_bytes -= best->second;
             d->kept.erase(best);
-            d->share();
             return cudaSuccess;
         }
     }
@@ -188,7 +215,10 @@ public:
     ~DevRelease()
     {
         current() = outer_;
-        if (sync_) cudaStreamSynchronize(pool_->stream);
+        try {
+            if (any_) pool_->balance(large_);
+        } catch (const std::bad_alloc &) {   // no room for its list: another release does it
+        }
     }
     DevRelease(const DevRelease &) = delete;
     DevRelease &operator=(const DevRelease &) = delete;
@@ -200,14 +230,16 @@ public:
         if (!r || r->pool_ != d) return wait_for_device();
         return r->waited_ = r->waited_ || wait_for_device();
     }
-    // a buffer went back, or the pool's share is smaller: what is above that goes when its stream is synchronized
-    static void released(DevPool *d)
+    // a small buffer went to pool d's stream, or a large one is kept
+    static void released(DevPool *d, bool large)
     {
         DevRelease *r = current();
-        if (r && r->pool_ == d)
-            r->sync_ = true;
-        else
-            cudaStreamSynchronize(d->stream);
+        if (r && r->pool_ == d) {
+            r->any_ = true;
+            r->large_ = r->large_ || large;
+        } else {
+            d->balance(large);
+        }
     }
 
 private:
@@ -218,7 +250,7 @@ private:
     }
     DevRelease *outer_;
     DevPool *pool_ = nullptr;
-    bool waited_ = false, sync_ = false;
+    bool waited_ = false, any_ = false, large_ = false;
 };
 
 // after all work of the memory's device
@@ -241,30 +273,27 @@ try {
         cudaGetLastError();   // a capture that forbids it or a failed context: the memory stays, since work may still read it
     } else {
         std::vector<std::pair<void *, size_t>> gone;   // given back outside the lock
-        bool large = false;
+        bool large = false, kept = false;
         {
             std::lock_guard<std::mutex> lock(d->mutex);
             const auto b = d->held.find(p);
             large = b != d->held.end();
             if (large) {
                 const std::pair<void *, size_t> buffer = *b;
-                d->held.erase(b);
-                size_t drop = 0;
-                if (buffer.second > kLargeKeep) {
-                    gone.push_back(buffer);
-                } else {
-                    while (d->kept_bytes + buffer.second > kLargeKeep) d->kept_bytes -= d->kept[drop++].second;
-                    gone.assign(d->kept.begin(), d->kept.begin() + drop);
-                    d->kept.erase(d->kept.begin(), d->kept.begin() + drop);
+                kept = buffer.second <= kLargeKeep;
+                if (kept) {
+                    d->drop(kLargeKeep - buffer.second, gone);
                     d->kept.push_back(buffer);
                     d->kept_bytes += buffer.second;
-                    d->share();
+                } else {
+                    gone.push_back(buffer);
                 }
+                d->held.erase(b);
             }
         }
         for (auto &b : gone) cudaFree(b.first);
         if (!large) cudaFreeAsync(p, d->stream);
-        DevRelease::released(d);
+        if (!large || kept) DevRelease::released(d, kept);
     }
     if (other) cudaSetDevice(cur);
 } catch (const std::bad_alloc &) {   // no room for the lists: the memory stays

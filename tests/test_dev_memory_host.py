@@ -20,7 +20,7 @@ RUNTIME = r'''
 #include <mutex>
 enum cudaError_t { cudaSuccess = 0, cudaErrorMemoryAllocation = 2, cudaErrorInvalidValue = 1, cudaErrorStreamCaptureUnsupported = 900 };
 enum { cudaDevAttrMemoryPoolsSupported, cudaMemAllocationTypePinned, cudaMemHandleTypeNone, cudaMemLocationTypeDevice,
-       cudaMemPoolAttrReleaseThreshold, cudaStreamNonBlocking };
+       cudaMemPoolAttrReleaseThreshold, cudaMemPoolAttrUsedMemCurrent, cudaMemPoolAttrReservedMemCurrent, cudaStreamNonBlocking };
 struct Fake {
     std::mutex m;
     size_t capacity = size_t(4) << 30, direct = 0, pooled = 0, unused = 0, pending = 0, threshold = 0;
@@ -48,6 +48,13 @@ inline cudaError_t cudaDeviceGetAttribute(int *v, int, int) { *v = fake().pools;
 inline cudaError_t cudaMemPoolCreate(cudaMemPool_t *p, const cudaMemPoolProps *) { *p = new int; return cudaSuccess; }
 inline cudaError_t cudaMemPoolDestroy(cudaMemPool_t) { return cudaSuccess; }
 inline cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, int, void *v) { fake().threshold = *static_cast<uint64_t *>(v); return cudaSuccess; }
+inline cudaError_t cudaMemPoolGetAttribute(cudaMemPool_t, int what, void *v)
+{
+    Fake &f = fake();
+    std::lock_guard<std::mutex> l(f.m);
+    *static_cast<uint64_t *>(v) = what == cudaMemPoolAttrReservedMemCurrent ? f.pooled : f.pooled - f.unused;
+    return cudaSuccess;
+}
 inline cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, int) { *s = new int; return cudaSuccess; }
 inline cudaError_t cudaMalloc(void **p, size_t n)
 {
@@ -154,6 +161,21 @@ int main(int, char **argv)
                 for (void *p : h) dev_free(p);
         }
         CHECK(f.pool_new <= 12);
+        void *big[3] = {get(290 * MB), get(290 * MB), get(290 * MB)};   // and after a large handle: its buffers make room
+        for (void *p : big) dev_free(p);
+        f.pool_new = 0;
+        for (int i = 0; i < 4; ++i) {
+            void *s[4][3];
+            for (auto &h : s)
+                for (void *&p : h) p = get(30 * MB);
+            for (auto &h : s)
+                for (void *p : h) dev_free(p);
+            CHECK(f.mapped() <= 1024 * MB + 256);
+        }
+        CHECK(f.pool_new <= 12);
+        void *a2 = get(290 * MB);
+        CHECK(f.mallocs == 6 && a2);   // the last released is still there
+        dev_free(a2);
     } else if (test("bound")) {   // at most 1 GiB stays, also of buffers that are each well below it, at once
         for (size_t n : {1 * MB, 30 * MB, 60 * MB, 250 * MB, 900 * MB}) {
             std::vector<void *> p;
